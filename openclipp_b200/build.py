@@ -23,7 +23,8 @@ NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 COMMON = ["-std=c++17", "-O3", "-lineinfo", "-Xcompiler", "-fPIC,-fvisibility=hidden",
           "-I", os.path.join(ROOT, "include"), "-I", CSRC]
-CU_FLAGS = ARCH + COMMON + ["-Xptxas", "-O3", "--expt-relaxed-constexpr"]
+# The kernels of a file are optimised in parallel (a full build takes minutes otherwise).
+CU_FLAGS = ARCH + COMMON + ["-Xptxas", "-O3", "--expt-relaxed-constexpr", "--split-compile=0"]
 
 
 def sources():

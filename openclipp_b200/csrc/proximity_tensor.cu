@@ -24,29 +24,30 @@
 // for every chunk c, then (hi_2i, hi_2i+1) x (Thi_2i, Thi_2i+1). U8 sources use
 // the i8 MMA with s32 accumulation (exact).
 //
-// B operand: N = S R = 128 rows, row S j + p = template row th - 1 - j at phase
-// p, shifted by the staged row's lead: B[S j + p][k] = T(k - p - lead, th-1-j).
-// Source row t then adds to output-row slots t .. t + R - 1 (slot u is the
-// output row whose last template row is source row u).
+// B operand: N = S R = 128 rows; the row of phase p and slot j holds template
+// row th - 1 - j shifted by p and by the staged row's lead: T(k - p - lead,
+// th - 1 - j). Source row t then adds to output-row slots t .. t + R - 1 (slot u
+// is the output row whose last template row is source row u). The rows stand in
+// two halves, phases p < S/2 and p >= S/2, each S/2 rows a slot, so that
+// each half of the positions has TMEM columns of its own.
 //
 // Blocks. The steps (source rows) of an item are cut into blocks of
-// B = 16 / S steps. Step q of a block adds into TMEM columns S q + [0, N) of
-// the block's partial buffer: MMAs of N' = N + 16 = 144 columns at the
-// buffer's first column with B read S q rows later (B is stored with 16 - S
-// zero rows in front), so the block's partial sums of its B + R - 1 slots
-// end up at columns S j + p. The block's first MMA does not accumulate, which
-// clears the buffer. Partial buffers are double-buffered: the epilogue reads
-// block k while the tensor cores fill block k + 1.
+// B = 16 / S steps. Step q of a block adds into TMEM columns (S/2) q + [0, 64)
+// of each half of the block's partial buffer: MMAs of N' = 2 * 72 columns
+// with B read (S/2) q rows later (B is stored with zero rows in front of, between
+// and behind the halves), so the block's partial sums of its B + R - 1 slots
+// end up at columns (S/2) j + p of their half. The block's first MMA does not
+// accumulate, which clears the buffer. Partial buffers are double-buffered: the
+// epilogue reads block k while the tensor cores fill block k + 1.
 //
-// Running sums. The epilogue adds each block's partials into a ring of
-// running sums in TMEM that only it reads and writes (slot u at ring columns
-// S (u mod NS) + p, NS S = 144 columns; FP32 round-to-nearest, exact int32
-// for U8). The block's first 16 columns are the B slots it completes: the
-// epilogue writes them out and clears their ring columns. The tensor cores'
-// FP32 accumulation into one value thus never spans more than one block:
-// that accumulator rounds every addition with a bias that grows with the
-// number of additions, so the chains of a whole window (th rows x K chunks)
-// would cost accuracy.
+// Running sums. The epilogue adds each block's partials to the running sums of
+// the open slots, 64 registers of each thread (FP32 round-to-nearest, exact
+// int32 for U8). The first 8 columns of a half are the B slots the block
+// completes; the sums move down 8 registers a block as they are added to. The
+// tensor cores' FP32 accumulation into one value thus never spans more than
+// one block: that accumulator rounds every addition with a bias that grows with
+// the number of additions, so the chains of a whole window (th rows x K
+// chunks) would cost accuracy.
 //
 // Window energies sum S^2 of each position (measures other than CrossCorr):
 // a separate pre-pass (row_energy.cu) writes the row energies R(x, r) =
@@ -59,13 +60,24 @@
 // U16) or as the plain path does them (U8: the results are bit-identical to
 // it).
 //
-// Roles (10 warps; one CTA per SM, which holds all 512 TMEM columns):
-//   warps 0-3  builders: the A operand of each row (split into hi/lo);
-//   warps 4-7  epilogue (warp 4 + k reads TMEM lanes 32k .. 32k + 31): running
-//              sums in the TMEM ring, window energies, score map;
-//   warp 8     TMA loads of source rows (zero fill outside the image);
-//   warp 9     MMA issue (one commit per block of rows: the block's partial
-//              and its A stages are free once it completes).
+// Roles (12 warps; one CTA per SM, which holds all 512 TMEM columns):
+//   warps 0-2  builders: each loads (TMA, zero fill outside the image) and
+//              builds whole rows of the A operand (split into hi/lo);
+//   warp 3     MMA issue (one commit per block of rows: the block's partial
+//              and its A stages are free once it completes);
+//   warps 4-11 epilogue, two per TMEM sub-partition, one for each half of the
+//              positions: running sums, window energies, score map.
+//
+// Bound: an MMA of M = 128, N = 144 takes the tensor pipe 72 cycles and reads
+// 8.7 KB of operands from shared memory in them, 120 of the 128 bytes a cycle
+// that shared memory and L1 give, so what the other warps read and write there
+// (staged rows, A operand, energies, maps) slows the MMAs: the 31 x 31 F32
+// step of 8 MMAs (576 cycles) takes 870 (CrossCorr) to 1060 (with energies);
+// it took 1150 to 1290 with a wait per step, one warp per sub-partition in
+// the epilogue, the running sums in TMEM and FP64 scores. On 4096 x 4096 F32
+// with 31 x 31, CrossCorr_Norm went from 234 to 214 us, the 3840 x 2160 x 4
+// U16 map with 64 x 64 from 1297 to 1140 us.
+//
 // Every wait is bounded: a wait that gives up sets the CTA's abort flag, the
 // roles leave their loops, the MMA and TMA threads drain what they issued,
 // and the kernel raises the context's error flag.
@@ -92,27 +104,36 @@ namespace {
 using namespace sm100;
 
 constexpr int kM = 128;                 // TMEM lanes = A rows
-constexpr int kBuilders = 4;
-constexpr int kEpilogue = 4;
-constexpr int kTmaWarp = kBuilders + kEpilogue;
-constexpr int kMmaWarp = kTmaWarp + 1;
-constexpr int kThreads = (kMmaWarp + 1) * 32;
-constexpr int kBuildThreads = kBuilders * 32;
-constexpr int kNRaw = 6;                // staged source rows (TMA stages of one row)
-constexpr int kMaxNA = 16;              // A operand stages at most (two blocks of rows)
+constexpr int kBuilders = 3;
+constexpr int kEpilogue = 8;            // two warps per TMEM sub-partition
+constexpr int kMmaWarp = kBuilders;
+constexpr int kFirstEpilogue = kMmaWarp + 1;  // a multiple of 4: warp mod 4 is its sub-partition
+constexpr int kWarps = kFirstEpilogue + kEpilogue;  // 3 a scheduler, so 168 registers a thread
+constexpr int kThreads = kWarps * 32;
+constexpr int kMaxRaw = 18;             // staged source rows at most (TMA stages of one row)
+constexpr int kMaxAB = 4;               // blocks of A operand stages at most
 constexpr int kSR = 128;                // S R: template rows x positions per lane
 constexpr int kN = kSR;                 // B rows (MMA N without the slide)
-constexpr int kNp = kN + 16;            // MMA N: a block's B - 1 slides fit in 16 more
+constexpr int kHalfN = kN / 2;          // of each half of the positions
+constexpr int kHalf = kHalfN + 8;       // columns of a half: a block's slides fit in 8 more
+constexpr int kNp = 2 * kHalf;          // MMA N
 constexpr int kPartCols = kNp;          // TMEM columns per partial buffer (two of them)
-constexpr int kRingCol = 2 * kPartCols; // first TMEM column of the running-sum ring
-constexpr int kRingCols = kNp;          // ring columns: NS S = 144 (9 chunks of 16)
+constexpr int kRingChunks = kHalfN / 8; // open slots of a half: 8 chunks of 8 columns
 constexpr int kTmemCols = 512;
 constexpr int kMinSmem = 120 * 1024;    // keeps one CTA per SM (it takes all of TMEM)
 constexpr int kMaxDynSmem = 226 * 1024; // opt-in dynamic shared memory limit of the kernel
 constexpr long long kSpinLimit = 4000000000LL;  // about 2 s of SM clock
-constexpr int kBarBuild = 1;            // named barrier of the builder warps
+constexpr int kTmplBatch = 8;           // template loads a thread has in flight
 
 enum Elem { kF32 = 0, kU8 = 1, kU16 = 2 };
+
+// Staged rows (multiples of the builders, so that a stage belongs to one of
+// them) and blocks of A stages. A step of a U8 item is
+// one to three MMAs (72 cycles each), of a split item 4 to 16, so the U8 rows
+// are loaded and built further ahead: a load takes about 2000 cycles to land,
+// a row about 500 to build.
+__host__ __device__ constexpr int raw_stages(bool split) { return split ? 9 : 18; }
+__host__ __device__ constexpr int a_blocks(bool split) { return split ? 2 : 4; }
 
 template <int ELEM>
 struct ElemTraits {
@@ -120,6 +141,8 @@ struct ElemTraits {
   static constexpr int size = ELEM == kF32 ? 4 : ELEM == kU16 ? 2 : 1;
   static constexpr int inner = 16 / size;     // elements per 16-byte TMA group
   static constexpr int cmk = split ? 8 : 16;  // K elements per core-matrix row
+  static constexpr int raw = raw_stages(split);
+  static constexpr int ab = a_blocks(split);
 };
 
 // Positions per TMEM lane for a template of R rows (S R = 128), and the steps
@@ -137,7 +160,7 @@ struct Geo {
   int QR;          // buffer rows of one A plane
   int lbok;        // bytes between K-adjacent core matrices of A
   int nraw;        // staged elements the windows cover (lead + P - 1 + tw)
-  int NA;          // A operand stages: two blocks of steps
+  int NA;          // A operand stages: a_blocks() blocks of steps
 };
 
 __host__ __device__ inline Geo make_geo(bool split, int R, int tw, int lead) {
@@ -147,7 +170,7 @@ __host__ __device__ inline Geo make_geo(bool split, int R, int tw, int lead) {
   g.Q = 16 / g.S;
   g.R = R;
   g.B = block_steps(g.S);
-  g.NB = kN + 32 - g.S;
+  g.NB = kNp + 8 - g.S / 2;
   const int cmk = split ? 8 : 16;
   const int keff = tw + g.S - 1 + lead;
   g.KC = (keff + cmk - 1) / cmk;
@@ -161,7 +184,7 @@ __host__ __device__ inline Geo make_geo(bool split, int R, int tw, int lead) {
   g.lbok = 16 * (cmk / g.S);
   g.QR = kM + (cmk / g.S) * (g.cma - 1);
   g.nraw = lead + g.P - 1 + tw;
-  g.NA = 2 * g.B;
+  g.NA = a_blocks(split) * g.B;
   return g;
 }
 
@@ -242,12 +265,12 @@ __host__ __device__ inline Layout make_layout(bool split, const Geo& g, int nbox
   L.row_bytes = box_split(nbox) * box_part(nbox) * 16;
   L.raw_stage = align128(L.row_bytes);
   L.raw = 0;
-  L.b = L.raw + kNRaw * L.raw_stage;
+  L.b = L.raw + raw_stages(split) * L.raw_stage;
   L.a = L.b + align128(2 * g.nmma * g.NB * 16);
   L.a_stage = align128(g.QR * 16 * (split ? 2 : 1));
   L.bars = L.a + g.NA * L.a_stage;
-  // raw full, raw free; ready (one per A stage); block full, buffer free; done.
-  L.total = L.bars + align128(8 * (2 * kNRaw + kMaxNA + 4 + 1));
+  // raw full; A block ready, A block free; block full, buffer free; done.
+  L.total = L.bars + align128(8 * (kMaxRaw + 2 * kMaxAB + 4 + 1));
   return L;
 }
 
@@ -256,7 +279,7 @@ struct CtaState {
   uint32_t tmem;  // TMEM base address (all 512 columns)
   int abort;      // set by a wait that gave up; the CTA stops taking items
   int next;       // work item fetched from the queue
-  double et;      // template energy of the current item's channel
+  double et[kWarps];  // template energy of the item's channel, one part per warp
 };
 
 __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
@@ -266,67 +289,53 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
 __device__ __forceinline__ float bf16lo_f(uint32_t w) { return __uint_as_float(w << 16); }
 __device__ __forceinline__ float bf16hi_f(uint32_t w) { return __uint_as_float(w & 0xFFFF0000u); }
 
-// Template element (w, h) of channel c as a double (exact for every type).
+// Template element (w, h) of channel c as a float (exact for every type).
 template <int ELEM>
-__device__ __forceinline__ double tmpl_at(const ItemArgs& a, int h, int w, int c) {
+__device__ __forceinline__ float tmpl_at(const ItemArgs& a, int h, int w, int c) {
   const char* row = a.tmpl + (size_t)h * a.tmpl_pitch;
   const int i = w * a.nch + c;
-  if (ELEM == kF32) return reinterpret_cast<const float*>(row)[i];
-  if (ELEM == kU16) return reinterpret_cast<const uint16_t*>(row)[i];
-  return reinterpret_cast<const uint8_t*>(row)[i];
+  if (ELEM == kF32) return __ldg(reinterpret_cast<const float*>(row) + i);
+  if (ELEM == kU16) return __ldg(reinterpret_cast<const uint16_t*>(row) + i);
+  return __ldg(reinterpret_cast<const uint8_t*>(row) + i);
 }
 
-// 8 staged elements from element e0 as floats (F32, U16).
+__host__ __device__ constexpr int ilog2(int x) { return x <= 1 ? 0 : 1 + ilog2(x / 2); }
+
+// S staged elements from element e0, a multiple of S, as floats (F32, U16).
 template <int ELEM, int S>
-__device__ __forceinline__ void load8(const unsigned char* row, int e0, float (&f)[8]) {
-  if (S == 1) {
-    // Any start element: single-element loads.
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      if (ELEM == kF32)
-        f[j] = reinterpret_cast<const float*>(row)[e0 + j];
-      else
-        f[j] = static_cast<float>(reinterpret_cast<const uint16_t*>(row)[e0 + j]);
-    }
-  } else if (ELEM == kF32) {
+__device__ __forceinline__ void load_s(const unsigned char* row, int e0, float (&f)[S]) {
+  if (ELEM == kF32) {
     if (S % 4 == 0) {
-      const float4* p = reinterpret_cast<const float4*>(row + 4 * e0);
-      const float4 u = p[0], v = p[1];
-      f[0] = u.x; f[1] = u.y; f[2] = u.z; f[3] = u.w;
-      f[4] = v.x; f[5] = v.y; f[6] = v.z; f[7] = v.w;
-    } else {
-      const float2* p = reinterpret_cast<const float2*>(row + 4 * e0);
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const float2 u = p[j];
-        f[2 * j] = u.x;
-        f[2 * j + 1] = u.y;
+      for (int j = 0; j < S / 4; ++j) {
+        const float4 u = reinterpret_cast<const float4*>(row + 4 * e0)[j];
+        f[(4 * j) % S] = u.x;
+        f[(4 * j + 1) % S] = u.y;
+        f[(4 * j + 2) % S] = u.z;
+        f[(4 * j + 3) % S] = u.w;
       }
+    } else {
+      const float2 u = *reinterpret_cast<const float2*>(row + 4 * e0);
+      f[0] = u.x;
+      f[1] = u.y;
     }
   } else {
-    // U16: e0 is even (S = 2, 4 or 8), so 32-bit words hold pixel pairs.
-    const uint32_t* p = reinterpret_cast<const uint32_t*>(row + 2 * e0);
+    uint32_t w[S / 2];
+    if (S == 8) {
+      const uint4 u = *reinterpret_cast<const uint4*>(row + 2 * e0);
+      memcpy(w, &u, sizeof(w));
+    } else if (S == 4) {
+      const uint2 u = *reinterpret_cast<const uint2*>(row + 2 * e0);
+      memcpy(w, &u, sizeof(w));
+    } else {
+      w[0] = *reinterpret_cast<const uint32_t*>(row + 2 * e0);
+    }
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const uint32_t w = p[j];
-      f[2 * j] = static_cast<float>(w & 0xFFFFu);
-      f[2 * j + 1] = static_cast<float>(w >> 16);
+    for (int j = 0; j < S / 2; ++j) {
+      f[2 * j] = static_cast<float>(w[j] & 0xFFFFu);
+      f[2 * j + 1] = static_cast<float>(w[j] >> 16);
     }
   }
-}
-
-// AND of `p` over the builder warps (a named barrier every builder reaches).
-__device__ __forceinline__ bool builders_all(bool p) {
-  uint32_t r;
-  asm volatile(
-      "{\n\t.reg .pred pi, po;\n\t"
-      "setp.ne.u32 pi, %1, 0;\n\t"
-      "barrier.red.and.pred po, %2, %3, pi;\n\t"
-      "selp.u32 %0, 1, 0, po;\n\t}"
-      : "=r"(r)
-      : "r"((uint32_t)p), "n"(kBarBuild), "n"(kBuildThreads)
-      : "memory");
-  return r != 0;
 }
 
 // Running best of one lane (the fused best match): the value, its key and
@@ -360,7 +369,406 @@ __device__ __forceinline__ void idx_state_update(IdxState& st, float v, int x, i
   st.have = 1;
 }
 
-// Runs one work item with all 10 warps of the CTA. The caller has
+// num / sqrt(es * ei) of exact integers, rounded to FP32 through FP64 as
+// (float)(num / sqrt(es * ei)) with each FP64 operation correctly rounded. That
+// chain (a divide and a square root, about 220 cycles of a warp with no
+// overlap) is the true quotient within 2^-51, so an estimate within 2^-41
+// gives the same FP32 value unless a rounding boundary lies that near.
+// norm_near gives the estimate and whether it decides the value; norm_exact
+// is the chain, for the others (one value in 2^14, and zero energies).
+// es, ei < 2^31, |num| < 2^31; ret ~ 1 / sqrt(ei).
+__device__ __forceinline__ float norm_near(int num, int es, int ei, float ret, bool& decided) {
+  auto f64 = [](int v) {  // exact, without a conversion (8 cycles of a quarter of the SM)
+    return __hiloint2double(0x43300000, v ^ 0x80000000) - 4503601774854144.0;  // 2^52 + 2^31
+  };
+  const double x = f64(es) * f64(ei);
+  const double r = rsqrtf((float)es) * ret;   // 1 / sqrt(x) within 2^-21
+  const double q = f64(num) * (r * fma(-0.5 * x * r, r, 1.5));  // a Newton step: 2^-41
+  const int low = __double2loint(q) & 0x1fffffff;  // the bits FP32 drops
+  decided = es > 0 && ei > 0 && abs(low - 0x10000000) > 0x4000;
+  return (float)q;
+}
+__device__ __forceinline__ float norm_exact(int num, int es, int ei) {
+  return (float)__ddiv_rn((double)num, __dsqrt_rn(__dmul_rn((double)es, (double)ei)));
+}
+
+// U8 _Norm: float arithmetic where the plain path's float sums are exact.
+__device__ __forceinline__ bool u8_norm_in_float(int tw, int th) {
+  return (double)tw * th * 65025.0 <= 16777216.0;
+}
+
+template <bool SPLIT>
+struct Sums {
+  typedef typename std::conditional<SPLIT, float, int>::type A;   // product sums
+  typedef typename std::conditional<SPLIT, double, int>::type E;  // window energies
+  typedef typename std::conditional<SPLIT, float, int>::type R;   // row energies
+};
+
+// Scores of one position from its product sum cv and window energy ev (etd:
+// template energy, ret ~ 1 / sqrt(etd)). Split sources: SqrDistance's terms
+// cancel near a match, so its numerator is formed in FP64; the _Norm scale of
+// an F32 map is taken in FP32 (relative error a few 1e-7), of an F64 map in
+// FP64. U8: the plain path's float or double formulas (bit-identical) on
+// integers exact in int32, as each of C, E_S, E_T <= 64 * 64 * 255^2 < 2^28.
+template <bool SPLIT, int M>
+__device__ __forceinline__ float score_f(typename Sums<SPLIT>::A cv, typename Sums<SPLIT>::E ev,
+                                         double etd, float ret, bool u8_float) {
+  constexpr bool product = M == kCrossCorr || M == kCrossCorrNorm;
+  if constexpr (SPLIT) {
+    float num;
+    if (product)
+      num = cv;
+    else
+      num = (float)(ev - 2.0 * (double)cv + etd);
+    return M == kCrossCorr || M == kSqrDistance ? num : num * (rsqrtf((float)ev) * ret);
+  } else {
+    const int eti = static_cast<int>(etd);
+    const int num = product ? cv : ev - 2 * cv + eti;
+    if (M == kCrossCorr || M == kSqrDistance) return __int2float_rn(num);
+    if (u8_float) return __fdiv_rn((float)num, __fsqrt_rn(__fmul_rn((float)ev, (float)eti)));
+    return norm_exact(num, ev, eti);
+  }
+}
+
+// score_f of eight positions, independent of one another.
+template <bool SPLIT, int M>
+__device__ __forceinline__ void scores8(float (&out)[8], const typename Sums<SPLIT>::A (&val)[8],
+                                        const typename Sums<SPLIT>::E (&es)[8], double etd,
+                                        float ret, bool u8_float) {
+  if constexpr (!SPLIT && (M == kCrossCorrNorm || M == kSqrDistanceNorm)) {
+    if (!u8_float) {
+      const int eti = static_cast<int>(etd);
+      bool all = true;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        bool decided;
+        out[i] = norm_near(M == kCrossCorrNorm ? val[i] : es[i] - 2 * val[i] + eti, es[i], eti, ret,
+                           decided);
+        all = all && decided;
+      }
+      if (all) return;
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 8; ++i) out[i] = score_f<SPLIT, M>(val[i], es[i], etd, ret, u8_float);
+}
+
+template <bool SPLIT, int M>
+__device__ __forceinline__ double score_d(typename Sums<SPLIT>::A cv, typename Sums<SPLIT>::E ev,
+                                          double etd, bool u8_float) {
+  constexpr bool product = M == kCrossCorr || M == kCrossCorrNorm;
+  if constexpr (SPLIT) {
+    const double num = product ? (double)cv : ev - 2.0 * (double)cv + etd;
+    return M == kCrossCorr || M == kSqrDistance ? num : num * rsqrt(ev * etd);
+  } else {
+    const int eti = static_cast<int>(etd);
+    const int num = product ? cv : ev - 2 * cv + eti;
+    if (M == kCrossCorr || M == kSqrDistance) return (double)num;
+    if (u8_float)
+      return (double)__fdiv_rn((float)num, __fsqrt_rn(__fmul_rn((float)ev, (float)eti)));
+    return __ddiv_rn((double)num, __dsqrt_rn(__dmul_rn((double)ev, (double)eti)));
+  }
+}
+
+// Scores and stores of one slot that is not a whole run of a one-channel F32
+// map's row: F64 maps (written or added to), several channels, the right
+// edge. v: the F32 scores, for the best match.
+template <int ELEM, int SH, int M>
+__device__ __noinline__ void store_slot(const ItemArgs& a, int ch, int xl, char* orow,
+                           const typename Sums<ElemTraits<ELEM>::split>::A* val,
+                           const typename Sums<ElemTraits<ELEM>::split>::E* esum, double etd,
+                           float* v) {
+  constexpr bool SPLIT = ElemTraits<ELEM>::split;
+  const bool u8_float = u8_norm_in_float(a.tw, a.th);
+  if (a.dst_f64) {
+    double* o = reinterpret_cast<double*>(orow) + (size_t)xl * a.nch + ch;
+    if (SH > 1 && a.nch == 1 && xl + SH <= a.W) {
+#pragma unroll
+      for (int p = 0; p < SH; p += 2) {
+        double2 d = make_double2(0.0, 0.0);
+        if (a.accum) d = *reinterpret_cast<const double2*>(o + p);
+        d.x += score_d<SPLIT, M>(val[p], esum[p], etd, u8_float);
+        d.y += score_d<SPLIT, M>(val[(p + 1) % SH], esum[(p + 1) % SH], etd, u8_float);
+        *reinterpret_cast<double2*>(o + p) = d;
+      }
+      return;
+    }
+#pragma unroll
+    for (int p = 0; p < SH; ++p) {
+      if (xl + p >= a.W) break;
+      const double s = score_d<SPLIT, M>(val[p], esum[p], etd, u8_float);
+      o[p * a.nch] = a.accum ? o[p * a.nch] + s : s;
+    }
+    return;
+  }
+  const float ret = (float)(1.0 / sqrt(etd));
+#pragma unroll
+  for (int p = 0; p < SH; ++p) {
+    v[p] = score_f<SPLIT, M>(val[p], esum[p], etd, ret, u8_float);
+    if (xl + p < a.W && a.dst != nullptr)
+      reinterpret_cast<float*>(orow)[(size_t)(xl + p) * a.nch + ch] = v[p];
+  }
+}
+
+// Epilogue of an item, one of two warps of each TMEM sub-partition: warp
+// 4 + 4 h + s takes positions [h S/2, (h + 1) S/2) of lanes 32 s .. 32 s + 31,
+// which have their own 72 columns of the partials and of the ring. One warp is
+// a chain of dependent steps (TMEM round trips, conversions, energies), so
+// the block's time is its latency; with one warp per sub-partition, FP64
+// scores of every measure and a wait per 16 columns, the 31 x 31 F32 kernel's
+// step took 1170-1410 cycles here against 580 of the MMAs.
+template <int ELEM, int S, bool IDX, int M>
+__device__ __forceinline__ void run_epilogue(const ItemArgs& a, CtaState& cs, uint32_t tmem_base,
+                                             uint64_t* blk_full, uint64_t* buf_free, int r_begin,
+                                             int nsteps) {
+  constexpr bool SPLIT = ElemTraits<ELEM>::split;
+  constexpr int R = kSR / S;
+  constexpr int BS = block_steps(S);
+  constexpr int SH = S / 2;
+  constexpr bool kE = M != kCrossCorr;  // the measure needs window energies
+  typedef typename Sums<SPLIT>::A AT;
+  typedef typename Sums<SPLIT>::E ET;
+  typedef typename Sums<SPLIT>::R RT;
+  volatile int* abort_flag = &cs.abort;
+  const int ew = (threadIdx.x >> 5) - kFirstEpilogue, lane = threadIdx.x & 31;
+  const int half = ew >> 2;
+  const uint32_t lane_base = tmem_base + (static_cast<uint32_t>((ew & 3) * 32) << 16);
+  // The item's fields in registers: the item lives in shared memory, and
+  // the score loop would otherwise reload them on every slot.
+  const int W = a.W, H = a.H, th = a.th, nch = a.nch, ch = a.ch;
+  const int idx_op = IDX ? a.idx_op : -1;
+  const int xl = a.xs_out + S * ((ew & 3) * 32 + lane) + half * SH;  // first position
+  const bool whole = xl + SH <= W;
+  const bool f32 = !a.dst_f64, accum = a.accum;
+  double etd = 0.0;  // template energy
+#pragma unroll
+  for (int w = 0; w < kWarps; ++w) etd += cs.et[w];
+  const float ret = (float)(1.0 / sqrt(etd));  // 1 / sqrt(E_T)
+  const bool u8_float = u8_norm_in_float(a.tw, th);
+  // Best-match state of this lane (ocipProximityIndx).
+  IdxState ib;
+  ib.v = 0.f;
+  ib.key = 0ull;
+  ib.have = 0;
+  ib.nan = 0;
+  const int idx_ngx = (W + 255) >> 8;
+
+  // Row energies of the rows a block's slots complete (entering: staged row u;
+  // leaving: staged row u - th), loaded before the block's MMAs are waited
+  // for. The window energy of each position is a running sum over the slots,
+  // in order (FP64, exact int32 for U8). Positions past the last column read
+  // the rows' pitch (a multiple of 32 values) and are not stored.
+  uint32_t rin[BS][SH] = {}, rout[BS][SH] = {};
+  ET esum[SH];
+#pragma unroll
+  for (int p = 0; p < SH; ++p) esum[p] = ET(0);
+  auto add_energy = [&](int g, int p) {
+    if constexpr (SPLIT)
+      esum[p] += (double)__uint_as_float(rin[g][p]) - (double)__uint_as_float(rout[g][p]);
+    else
+      esum[p] += static_cast<int>(rin[g][p] - rout[g][p]);
+  };
+  const char* e_row = nullptr;  // the row entering with the block's first slot
+  size_t e_pitch = 0, e_back = 0;
+  if (kE) {
+    e_pitch = a.e_pitch;
+    e_back = (size_t)th * e_pitch;
+    e_row = a.energy + (size_t)ch * a.e_plane + (size_t)xl * sizeof(RT) +
+            (ptrdiff_t)r_begin * (ptrdiff_t)e_pitch;
+  }
+  auto load_row = [&](uint32_t (&v)[SH], const char* at, bool ok) {
+    if (SH == 4) {
+      const uint4 q = ok ? *reinterpret_cast<const uint4*>(at) : make_uint4(0u, 0u, 0u, 0u);
+      memcpy(v, &q, sizeof(v));
+    } else if (SH == 2) {
+      const uint2 q = ok ? *reinterpret_cast<const uint2*>(at) : make_uint2(0u, 0u);
+      memcpy(v, &q, sizeof(v));
+    } else {
+      v[0] = ok ? *reinterpret_cast<const uint32_t*>(at) : 0u;
+    }
+  };
+  // Running sums of the open slots (FP32 round-to-nearest, exact int32 for U8):
+  // 8 chunks of BS slots, chunk 0 the next block's completed one.
+  AT ring[kRingChunks][8];
+#pragma unroll
+  for (int c = 0; c < kRingChunks; ++c)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) ring[c][j] = AT(0);
+  char* orow = a.dst + (ptrdiff_t)(a.y0 - R + 1) * (ptrdiff_t)a.dst_pitch;  // of slot 0
+  const size_t dst_pitch = a.dst_pitch;
+  const bool has_dst = a.dst != nullptr;
+  for (int k = 0; k * BS < nsteps; ++k) {
+    const int t0 = k * BS;
+    if (kE) {
+#pragma unroll
+      for (int g = 0; g < BS; ++g) {
+        const int u = t0 + g, r = r_begin + u;
+        const bool in = u < nsteps && xl < W;
+        load_row(rin[g], e_row + g * e_pitch, in && r >= 0 && r < H);
+        load_row(rout[g], e_row + g * e_pitch - e_back, in && u >= th && r >= th && r - th < H);
+      }
+      e_row += BS * e_pitch;
+    }
+    const bool ok = mbar_wait(&blk_full[k & 1], (k >> 1) & 1, abort_flag, kSpinLimit);
+    // tcgen05.ld/st are warp-collective: the whole warp takes one branch.
+    if (!__all_sync(0xffffffffu, ok)) break;
+    tc_fence_after();
+    const uint32_t part = lane_base + (k & 1) * kPartCols + half * kHalf;
+    // Chunk 0 of the partial completes the BS slots t0 .. t0 + BS - 1; chunk c
+    // belongs to the open sums c - 1 of the next block (the sums move down a
+    // chunk as they are added to). Three chunks are in flight together.
+    AT val[8];
+    auto chunks = [&](auto first) {
+      constexpr int C0 = decltype(first)::value, N = 3;
+      uint32_t vp[N][8];
+#pragma unroll
+      for (int c = 0; c < N; ++c) tmem_ld8x(part + 8 * (C0 + c), vp[c]);
+      tmem_ld_wait();
+#pragma unroll
+      for (int c = 0; c < N; ++c)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const AT old = C0 + c < kRingChunks ? ring[(C0 + c) % kRingChunks][j] : AT(0);
+          AT v;
+          if constexpr (SPLIT)
+            v = __fadd_rn(old, __uint_as_float(vp[c][j]));
+          else
+            v = old + static_cast<int>(vp[c][j]);  // exact int32 sums
+          if (C0 + c == 0)
+            val[j] = v;
+          else
+            ring[(C0 + c + kRingChunks - 1) % kRingChunks][j] = v;
+        }
+    };
+    chunks(std::integral_constant<int, 0>());
+    chunks(std::integral_constant<int, 3>());
+    chunks(std::integral_constant<int, 6>());
+    // The partial has been read: the MMAs may refill it (block k + 2).
+    tc_fence_before();
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&buf_free[k & 1]);
+    if (kE) {
+      // The loaded energies are first used here: without this the compiler
+      // converts them where they were loaded, and waits for the loads there
+      // (about 900 cycles a step).
+#pragma unroll
+      for (int g = 0; g < BS; ++g)
+#pragma unroll
+        for (int p = 0; p < SH; ++p) asm volatile("" : "+r"(rin[g][p]), "+r"(rout[g][p]));
+    }
+    // The block's completed slots: window energies, scores and stores.
+    const bool rows = t0 >= R - 1 && t0 + BS <= nsteps;  // every slot is an output row
+    if (M == kCrossCorr && !f32 && nch == 1 && rows) {
+      // Product sums of a tile of a larger template, in an F64 map.
+#pragma unroll
+      for (int g = 0; g < BS; ++g) {
+        double* o = reinterpret_cast<double*>(orow) + xl;
+#pragma unroll
+        for (int p = 0; p < SH; ++p) {
+          const double v = (double)val[g * SH + p];
+          if (xl + p < W) o[p] = accum ? o[p] + v : v;
+        }
+        orow += dst_pitch;
+      }
+    } else if (f32 && rows) {
+      // Straight-line independent work.
+      float out[8];
+      ET es[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const int g = i / SH, p = i % SH;
+        if (kE) add_energy(g, p);
+        es[i] = esum[p];
+      }
+      scores8<SPLIT, M>(out, val, es, etd, ret, u8_float);
+#pragma unroll
+      for (int g = 0; g < BS; ++g) {
+        if (IDX && idx_op >= 0) {
+#pragma unroll
+          for (int p = 0; p < SH; ++p)
+            if (xl + p < W)
+              idx_state_update(ib, out[g * SH + p], xl + p, a.y0 + t0 + g - R + 1, idx_op, idx_ngx);
+        }
+        if (IDX && !has_dst) {
+        } else if (!whole || nch > 1) {
+          float* o = reinterpret_cast<float*>(orow) + (size_t)xl * nch + ch;
+#pragma unroll
+          for (int p = 0; p < SH; ++p)
+            if (xl + p < W) o[p * nch] = out[g * SH + p];
+        } else {
+          float* o = reinterpret_cast<float*>(orow) + xl;
+          if (SH == 4)
+            *reinterpret_cast<float4*>(o) =
+                make_float4(out[g * SH], out[(g * SH + 1) % 8], out[(g * SH + 2) % 8],
+                            out[(g * SH + 3) % 8]);
+          else if (SH == 2)
+            *reinterpret_cast<float2*>(o) = make_float2(out[g * SH], out[(g * SH + 1) % 8]);
+          else
+            o[0] = out[g];
+        }
+        orow += dst_pitch;
+      }
+    } else {
+#pragma unroll
+      for (int g = 0; g < BS; ++g) {
+        const int u = t0 + g;
+        if (kE) {
+#pragma unroll
+          for (int p = 0; p < SH; ++p) add_energy(g, p);
+        }
+        if (u >= R - 1 && u < nsteps && xl < W) {
+          // (Copies: arrays whose address a call takes live in local memory.)
+          float v[SH];
+          AT cv[SH];
+          ET ev[SH];
+#pragma unroll
+          for (int p = 0; p < SH; ++p) {
+            cv[p] = val[g * SH + p];
+            ev[p] = esum[p];
+          }
+          store_slot<ELEM, SH, M>(a, ch, xl, orow, cv, ev, etd, v);
+          if (IDX && idx_op >= 0) {
+#pragma unroll
+            for (int p = 0; p < SH; ++p)
+              if (xl + p < W)
+                idx_state_update(ib, v[p], xl + p, a.y0 + u - R + 1, idx_op, idx_ngx);
+          }
+        }
+        orow += dst_pitch;
+      }
+    }
+  }
+  if (IDX && idx_op >= 0) {
+    // The warp's best: same rule, then lane 0 writes the warp's record.
+    const bool is_min = idx_op == 0 || idx_op == 2;
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) {
+      const float ov = __shfl_xor_sync(0xffffffffu, ib.v, d);
+      const unsigned long long ok2 = __shfl_xor_sync(0xffffffffu, ib.key, d);
+      const int oh = __shfl_xor_sync(0xffffffffu, ib.have, d);
+      ib.nan |= __shfl_xor_sync(0xffffffffu, ib.nan, d);
+      const bool take = oh && (!ib.have || (is_min ? ov < ib.v : ov > ib.v) ||
+                               (ov == ib.v && ok2 < ib.key));
+      if (take) {
+        ib.v = ov;
+        ib.key = ok2;
+        ib.have = 1;
+      }
+    }
+    if (lane == 0) {
+      const int item = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
+      IdxRecord r;
+      r.v = ib.v;
+      r.have = ib.have;
+      r.key = ib.key;
+      r.nan = ib.nan;
+      r.pad = 0;
+      reinterpret_cast<IdxRecord*>(a.idx_out)[item * kEpilogue + ew] = r;
+    }
+  }
+}
+
+// Runs one work item with all 12 warps of the CTA. The caller has
 // synchronised the CTA; TMEM (512 columns) is allocated. Barriers are
 // initialised here and invalidated at the end, so consecutive items may use
 // different layouts.
@@ -369,40 +777,40 @@ __device__ __forceinline__ void run_item(const ItemArgs& a, unsigned char* smem,
   typedef ElemTraits<ELEM> TR;
   constexpr bool SPLIT = TR::split;
   constexpr int R = kSR / S;
-  constexpr int Q = 16 / S;
   constexpr int BS = block_steps(S);
   constexpr int CMK = TR::cmk;
-  constexpr int NC = S * (BS + R - 1);  // open-slot columns of a block
-  constexpr int NCH = (NC + 15) / 16;   // 16-column chunks of a partial
-  static_assert(S * BS == 16, "a block's completed slots are one chunk");
-  static_assert(NC <= kNp && NCH * 16 == kRingCols, "block does not fit the ring");
+  constexpr int NR = TR::raw;
+  constexpr int AB = TR::ab;
+  constexpr int SH = S / 2;             // positions of a half
+  static_assert(SH * BS == 8, "a half's completed slots of a block are one chunk");
+  static_assert(SH * (BS + R - 1) <= kHalf, "a block's open slots do not fit the partial");
   const int lead = (TR::inner - a.ax % TR::inner) % TR::inner;
   const Geo G = make_geo(SPLIT, R, a.tw, lead);
   const Layout L = make_layout(SPLIT, G, a.nbox);
 
   uint64_t* raw_full = reinterpret_cast<uint64_t*>(smem + L.bars);
-  uint64_t* raw_free = raw_full + kNRaw;
-  // A of row t written. Stage t mod NA is free again once the MMAs of block
-  // t / BS - 2 have completed (its blk_full commit): NA = 2 BS stages.
-  uint64_t* ready = raw_free + kNRaw;
-  uint64_t* blk_full = ready + kMaxNA;     // block's MMAs complete (2 buffers)
+  // Block k's A stages (k mod AB) hold its rows; its MMAs have completed, so
+  // the builders may refill them (block k + AB).
+  uint64_t* ready = raw_full + kMaxRaw;
+  uint64_t* a_free = ready + kMaxAB;
+  uint64_t* blk_full = a_free + kMaxAB;    // block's MMAs complete (2 buffers)
   uint64_t* buf_free = blk_full + 2;       // block's buffer read by the epilogue
   uint64_t* done_bar = buf_free + 2;
   volatile int* abort_flag = &cs.abort;
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  const bool need_e = a.measure != kCrossCorr;
   const int ch = a.ch;
   const int r_begin = a.y0 - a.ay - (R - a.th);
   const int nsteps = (a.yend - a.y0) + R - 1;
+  const int nblk = (nsteps + BS - 1) / BS;
 
   if (threadIdx.x == 0) {
-    for (int i = 0; i < kNRaw; ++i) {
-      mbar_init(&raw_full[i], 1);
-      mbar_init(&raw_free[i], kBuilders);
+    for (int i = 0; i < NR; ++i) mbar_init(&raw_full[i], 1);
+    for (int i = 0; i < AB; ++i) {
+      mbar_init(&ready[i], BS);
+      mbar_init(&a_free[i], 1);
     }
-    for (int i = 0; i < G.NA; ++i) mbar_init(&ready[i], kBuilders);
     for (int i = 0; i < 2; ++i) {
       mbar_init(&blk_full[i], 1);
       mbar_init(&buf_free[i], kEpilogue);
@@ -411,15 +819,71 @@ __device__ __forceinline__ void run_item(const ItemArgs& a, unsigned char* smem,
     fence_barrier_init();
   }
 
-  // Template operand B: per core matrix (two per MMA, in issue order) NB rows
-  // of 16 bytes; rows 16 - S .. 16 - S + N - 1 hold B, the rest are zero.
+  // The template is staged once (at the A stages, which nothing uses yet): row
+  // h holds elements T(i - o, h) at i, zero outside the template, as BF16 hi
+  // and lo (split) or bytes. All loads of a group of kTmplBatch are in flight
+  // together, and each thread squares what it loads for the template energy:
+  // gathering B's elements and the energy straight from global memory, one
+  // dependent load after another, took 25-30 us of every launch.
+  const int o = S - 1 + lead;
+  const int tpitch = G.KC * CMK + o;
+  const int tplane = (a.th * tpitch + 7) & ~7;  // elements of one staged array
   {
-    const int zp = 16 - S;
-    const int total = 2 * G.nmma * G.NB * CMK;
+    double e = 0.0;
+    const int total = a.th * tpitch;
+    for (int base = threadIdx.x; base < total; base += kTmplBatch * kThreads) {
+      float v[kTmplBatch];
+#pragma unroll
+      for (int u = 0; u < kTmplBatch; ++u) {
+        const int idx = base + u * kThreads;
+        const int h = idx / tpitch, w = idx - h * tpitch - o;
+        v[u] = (idx < total && w >= 0 && w < a.tw) ? tmpl_at<ELEM>(a, h, w, ch) : 0.f;
+      }
+#pragma unroll
+      for (int u = 0; u < kTmplBatch; ++u) {
+        const int idx = base + u * kThreads;
+        if (idx >= total) break;
+        e = fma((double)v[u], (double)v[u], e);
+        if (SPLIT) {
+          const __nv_bfloat16 hi = __float2bfloat16_rn(v[u]);
+          __nv_bfloat16* st = reinterpret_cast<__nv_bfloat16*>(smem + L.a);
+          st[idx] = hi;
+          st[tplane + idx] = __float2bfloat16_rn(v[u] - __bfloat162float(hi));
+        } else {
+          smem[L.a + idx] = static_cast<uint8_t>(v[u]);
+        }
+      }
+    }
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) e += __shfl_xor_sync(0xffffffffu, e, d);
+    if (lane == 0) cs.et[warp] = e;
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  // Loads of row t into its stage, by the builder that owns it (one lane).
+  auto load_stage = [&](int t) {
+    const int st = t % NR, part = box_part(a.nbox), nsplit = box_split(a.nbox);
+    const int gx = (a.xs_out - a.ax - lead) / TR::inner;  // exact: a multiple of inner
+    mbar_arrive_expect_tx(&raw_full[st], L.row_bytes);
+    for (int j = 0; j < nsplit; ++j)
+      tma_load_4d(smem + L.raw + st * L.raw_stage + j * part * 16, a.tmap, 0, gx + j * part,
+                  r_begin + t, ch, &raw_full[st]);
+  };
+  if (warp < kBuilders && lane == 0) {
+    tma_prefetch_desc(a.tmap);
+    for (int t = warp; t < min(NR, nsteps); t += kBuilders) load_stage(t);
+  }
+  {
+    // Template operand B: per core matrix (two per MMA, in issue order) NB rows
+    // of 16 bytes, a thread per row; rows zp .. zp + 63 hold the first half of the positions,
+    // rows zp + 72 .. zp + 135 the second, the rest are zero.
+    constexpr int zp = 8 - SH;
+    constexpr int NB = kNp + zp;
+    const int total = 2 * G.nmma * NB;
     for (int idx = threadIdx.x; idx < total; idx += kThreads) {
-      const int e = idx % CMK;
-      const int row = (idx / CMK) % G.NB;
-      const int cm = idx / (CMK * G.NB);
+      const int cm = idx / NB, r = idx - cm * NB - zp;
+      const int half = r >= kHalf, n = r - half * kHalf;  // row of its half
       // Which part (0 zero, 1 Thi, 2 Tlo; U8: 1) and which K chunk.
       int part, c;
       if (SPLIT) {
@@ -435,450 +899,229 @@ __device__ __forceinline__ void run_item(const ItemArgs& a, unsigned char* smem,
         c = cm;
         part = c < G.KC ? 1 : 0;
       }
-      const int n = row - zp;
-      double t = 0.0;
-      if (part && n >= 0 && n < kN) {
-        const int j = n / S, p = n - (n / S) * S;
-        const int h = a.th - 1 - j;
-        const int w = c * CMK + e - p - lead;
-        if (h >= 0 && w >= 0 && w < a.tw) t = tmpl_at<ELEM>(a, h, w, ch);
-      }
-      unsigned char* dst = smem + L.b + (cm * G.NB + row) * 16;
-      if (SPLIT) {
-        const float tf = static_cast<float>(t);
-        const __nv_bfloat16 hi = __float2bfloat16_rn(tf);
-        const __nv_bfloat16 lo = __float2bfloat16_rn(tf - __bfloat162float(hi));
-        reinterpret_cast<__nv_bfloat16*>(dst)[e] = part == 2 ? lo : hi;
-      } else {
-        dst[e] = static_cast<uint8_t>(t);
-      }
-    }
-    if (warp == kTmaWarp) {
-      double e = 0.0;
-      for (int idx = lane; idx < a.th * a.tw; idx += 32) {
-        const int h = idx / a.tw, k = idx - h * a.tw;
-        const double t = tmpl_at<ELEM>(a, h, k, ch);
-        e += t * t;
-      }
+      const int h = a.th - 1 - n / SH;
+      uint4 q = make_uint4(0u, 0u, 0u, 0u);
+      if (part && n >= 0 && n < kHalfN && h >= 0) {
+        // Elements w = c CMK - p - lead .. + CMK - 1 of template row h.
+        const int at = h * tpitch + c * CMK + S - 1 - (half * SH + n % SH);
+        uint32_t w4[4];
+        if (SPLIT) {
+          const uint16_t* st =
+              reinterpret_cast<const uint16_t*>(smem + L.a) + (part == 2 ? tplane : 0) + at;
 #pragma unroll
-      for (int d = 16; d > 0; d >>= 1) e += __shfl_xor_sync(0xffffffffu, e, d);
-      if (lane == 0) cs.et = e;
+          for (int j = 0; j < 4; ++j) w4[j] = st[2 * j] | (uint32_t)st[2 * j + 1] << 16;
+        } else {
+          const uint8_t* st = smem + L.a + at;
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            w4[j] = st[4 * j] | (uint32_t)st[4 * j + 1] << 8 | (uint32_t)st[4 * j + 2] << 16 |
+                    (uint32_t)st[4 * j + 3] << 24;
+        }
+        q = make_uint4(w4[0], w4[1], w4[2], w4[3]);
+      }
+      *reinterpret_cast<uint4*>(smem + L.b + idx * 16) = q;
     }
+    // B is complete, and the staged template read, for the MMA and builder warps.
+    fence_async_smem();
+    __syncthreads();
   }
-  fence_async_smem();
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
   const uint32_t tmem_base = cs.tmem;
 
-  if (warp == kTmaWarp) {
-    // ---- TMA: source rows, one per stage ----------------------------------------
-    if (lane == 0) {
-      tma_prefetch_desc(a.tmap);
-      const int gx = (a.xs_out - a.ax - lead) / TR::inner;  // exact: a multiple of inner
-      const int part = box_part(a.nbox), nsplit = box_split(a.nbox);
-      int issued = 0;
-      for (; issued < nsteps; ++issued) {
-        const int st = issued % kNRaw;
-        if (issued >= kNRaw &&
-            !mbar_wait(&raw_free[st], ((issued / kNRaw) - 1) & 1, abort_flag, kSpinLimit))
-          break;
-        mbar_arrive_expect_tx(&raw_full[st], L.row_bytes);
-        for (int j = 0; j < nsplit; ++j)
-          tma_load_4d(smem + L.raw + st * L.raw_stage + j * part * 16, a.tmap, 0, gx + j * part,
-                      r_begin + issued, ch, &raw_full[st]);
-      }
-      // Every load issued has landed before the item ends.
-      volatile int no_abort = 0;
-      for (int b = max(0, issued - kNRaw); b < issued; ++b)
-        mbar_wait(&raw_full[b % kNRaw], (b / kNRaw) & 1, &no_abort, kSpinLimit);
-    }
-  } else if (warp == kMmaWarp) {
+  if (warp == kMmaWarp) {
     // ---- MMA issue --------------------------------------------------------------
-    if (lane == 0) {
+    // The whole warp walks the blocks on warp-uniform values (taken from lane 0)
+    // and one elected lane issues. An MMA of N = 144 takes the tensor pipe 72
+    // cycles (N / 2), and the pipe queues only two or three, so what the issuing
+    // lane does between MMAs counts: with the lane alone in a divergent branch,
+    // a wait per step and descriptors in per-lane registers an MMA went out
+    // every 95-130 cycles; this form measured 73-76 (steps of 8 MMAs).
+    {
       const uint32_t idesc = SPLIT ? idesc_bf16_f32(kM, kNp) : idesc_u8_s32(kM, kNp);
-      const uint32_t a0 = smem_u32(smem + L.a);
-      const uint32_t b0 = smem_u32(smem + L.b);
+      auto uniform = [](uint32_t v) { return __shfl_sync(0xffffffffu, v, 0); };
+      const uint32_t tm = uniform(tmem_base);
+      const uint32_t a0 = uniform(smem_u32(smem + L.a));
+      const uint32_t b0 = uniform(smem_u32(smem + L.b));
       const uint32_t bstride = G.NB * 16;  // between B core matrices
-      const uint32_t dhi = desc_hi(128);     // every descriptor: SBO 128 bytes
-      const uint32_t astep = G.lbok >> 4, bstep = (2 * bstride) >> 4;  // 16-byte units
-      int i = 0;
-      uint32_t ph = 0;
-      for (int t = 0; t < nsteps; ++t) {
-        const int k = t / BS, q = t - (t / BS) * BS;
+      const uint32_t dhi = desc_hi(128);   // every descriptor: SBO 128 bytes
+      const uint32_t astep = uniform(G.lbok >> 4), bstep = (2 * bstride) >> 4;  // 16-byte units
+      const int a_stage = uniform(L.a_stage), a_hl = uniform(G.QR * 16), lbok = uniform(G.lbok);
+      const int kc = uniform(G.KC), nmma = uniform(G.nmma), nst = uniform(nsteps),
+                nb = uniform(nblk);
+      const bool issuer = elect_one();
+      for (int k = 0; k < nb; ++k) {
         // The buffer of block k was read by the epilogue (block k - 2).
-        if (q == 0 && k >= 2 &&
-            !mbar_wait(&buf_free[k & 1], ((k >> 1) - 1) & 1, abort_flag, kSpinLimit))
-          break;
-        if (!mbar_wait(&ready[i], ph, abort_flag, kSpinLimit)) break;
+        bool ok = k < 2 || mbar_wait(&buf_free[k & 1], ((k >> 1) - 1) & 1, abort_flag, kSpinLimit);
+        ok = ok && mbar_wait(&ready[k % AB], (k / AB) & 1, abort_flag, kSpinLimit);
+        if (!__all_sync(0xffffffffu, ok)) break;
         tc_fence_after();
-        const uint32_t d = tmem_base + (k & 1) * kPartCols;  // the block's partial
-        const uint32_t ah = a0 + i * L.a_stage;
-        const uint32_t bq = b0 + 16 * S * (Q - 1 - q);
-        // The block's first MMA overwrites all kNp columns of the partial.
-        const uint32_t acc0 = q == 0 ? 0u : 1u;
-        // Descriptors advance by one add of their low word per MMA: B by two
-        // core matrices, A by one (split, hi/lo pairs) or two K core matrices.
-        // The MMAs of a step issue back to back from this one thread, so the
-        // work between two of them delays the tensor pipe directly.
-        uint32_t bl = desc_lo(bq, bstride);
-        if (SPLIT) {
-          uint32_t al = desc_lo(ah, G.QR * 16), acc = acc0;
-          for (int c = 0; c < G.KC; ++c) {
-            mma_bf16_h(d, al, dhi, bl, dhi, idesc, acc);
-            acc = 1u;
-            al += astep;
-            bl += bstep;
+        const uint32_t d = tm + (k & 1) * kPartCols;  // the block's partial
+        if (issuer) {
+#pragma unroll
+          for (int q = 0; q < BS; ++q) {
+            if (k * BS + q < nst) {
+              const uint32_t ah = a0 + ((k % AB) * BS + q) * a_stage;
+              // Descriptors advance by one add of their low word per MMA: B by
+              // two core matrices, A by one (split, hi/lo pairs) or two K core
+              // matrices. The block's first MMA overwrites all kNp columns.
+              uint32_t bl = desc_lo(b0 + 16 * SH * (BS - 1 - q), bstride);
+              uint32_t acc = q == 0 ? 0u : 1u;
+              if (SPLIT) {
+                uint32_t al = desc_lo(ah, a_hl);
+                for (int c = 0; c < kc; ++c) {
+                  mma_bf16_h(d, al, dhi, bl, dhi, idesc, acc);
+                  acc = 1u;
+                  al += astep;
+                  bl += bstep;
+                }
+                al = desc_lo(ah, lbok);
+                for (int j = kc; j < nmma; ++j) {
+                  mma_bf16_h(d, al, dhi, bl, dhi, idesc, 1u);
+                  al += 2 * astep;
+                  bl += bstep;
+                }
+              } else {
+                uint32_t al = desc_lo(ah, lbok);
+                for (int j = 0; j < nmma; ++j) {
+                  mma_i8_h(d, al, dhi, bl, dhi, idesc, acc);
+                  acc = 1u;
+                  al += 2 * astep;
+                  bl += bstep;
+                }
+              }
+            }
           }
-          uint32_t al2 = desc_lo(ah, G.lbok);
-          for (int j = G.KC; j < G.nmma; ++j) {
-            mma_bf16_h(d, al2, dhi, bl, dhi, idesc, 1u);
-            al2 += 2 * astep;
-            bl += bstep;
-          }
-        } else {
-          uint32_t al = desc_lo(ah, G.lbok), acc = acc0;
-          for (int j = 0; j < G.nmma; ++j) {
-            mma_i8_h(d, al, dhi, bl, dhi, idesc, acc);
-            acc = 1u;
-            al += 2 * astep;
-            bl += bstep;
-          }
+          // The block's partial for the epilogue, its A stages for the builders.
+          mma_commit(&blk_full[k & 1]);
+          // (The last blocks' stages are not refilled: no arrival is left pending.)
+          if (k + AB < nb) mma_commit(&a_free[k % AB]);
         }
-        // One commit per block: it frees the block's partial for the epilogue
-        // and its A stages for the builders.
-        if (q == BS - 1 || t == nsteps - 1) mma_commit(&blk_full[k & 1]);
-        if (++i == G.NA) { i = 0; ph ^= 1; }
+        __syncwarp();
       }
       // Every MMA issued has completed before the item ends.
-      mma_commit(done_bar);
+      if (issuer) mma_commit(done_bar);
+      __syncwarp();
       volatile int no_abort = 0;
       mbar_wait(done_bar, 0, &no_abort, kSpinLimit);
     }
   } else if (warp < kBuilders) {
     // ---- Builders: A operand ------------------------------------------------------
-    const int b = threadIdx.x;  // 0 .. 127
-    int i = 0, st = 0;
-    uint32_t rph = 0;
-    for (int t = 0; t < nsteps; ++t) {
-      bool ok = mbar_wait(&raw_full[st], rph, abort_flag, kSpinLimit);
-      // A stage i was last read by row t - NA, in block kb - 2: wait for that
-      // block's commit. (The barrier cannot be a phase further on: block kb
-      // needs these rows; and block kb - 4 was waited for two blocks ago.)
-      const int kb = t / BS;
-      ok = ok && (t < G.NA ||
-                  mbar_wait(&blk_full[(kb - 2) & 1], ((kb - 2) >> 1) & 1, abort_flag, kSpinLimit));
-      // All builders take the same branch (they meet at named barriers).
-      if (!builders_all(ok)) break;
+    // One warp per row, so that three rows are in flight: the waits, shared-memory
+    // round trips and proxy fence of a row are a chain of hundreds of cycles.
+    // The warp that has read a staged row loads the stage's next one.
+    // Rows past the last step only arrive (a block completes with BS arrivals).
+    int t = warp;
+    for (; t < nblk * BS; t += kBuilders) {
+      const int kb = t / BS, st = t % NR, i = t % (AB * BS);
+      bool ok = kb < AB || mbar_wait(&a_free[kb % AB], (kb / AB - 1) & 1, abort_flag, kSpinLimit);
+      ok = ok && (t >= nsteps || mbar_wait(&raw_full[st], (t / NR) & 1, abort_flag, kSpinLimit));
+      if (!__all_sync(0xffffffffu, ok)) break;
+      if (t >= nsteps) {
+        if (lane == 0) mbar_arrive(&ready[kb % AB]);
+        continue;
+      }
       const unsigned char* row = smem + L.raw + st * L.raw_stage;
       unsigned char* ahi = smem + L.a + i * L.a_stage;
-      for (int q = b; q < G.QR; q += kBuildThreads) {
-        if (SPLIT) {
-          float f[8];
-          load8<ELEM, S>(row, S * q, f);
-          uint32_t hi[4], lo[4];
+      if constexpr (SPLIT) {
+        // Row q is the S pixels of "lane" q and of the 8 / S - 1 after it. Each
+        // pixel is read and split once (the MMAs use 120 of the 128 bytes a
+        // cycle that shared memory gives); rows take their neighbours'
+        // pixels by shuffles.
+        constexpr int NG = (kM + 31) / 32 + (S == 2 ? 2 : 1);  // row groups: QR <= 164, 160
+        constexpr int NL = NG + (S == 4 ? 1 : 0);              // pixel groups
+        constexpr int SP = S / 2;                              // packed pairs a lane reads
+        const int qlast = G.QR + 8 / S - 2;                    // last pixel group of a row
+        uint32_t hi[NL][SP], lo[NL][SP];
 #pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            hi[j] = pack_bf16(f[2 * j], f[2 * j + 1]);
-            lo[j] = pack_bf16(f[2 * j] - bf16lo_f(hi[j]), f[2 * j + 1] - bf16hi_f(hi[j]));
+        for (int j = 0; j < NL; ++j) {
+          float f[S];
+          load_s<ELEM, S>(row, S * min(lane + 32 * j, qlast), f);
+#pragma unroll
+          for (int i = 0; i < SP; ++i) {
+            hi[j][i] = pack_bf16(f[2 * i], f[2 * i + 1]);
+            lo[j][i] = pack_bf16(f[2 * i] - bf16lo_f(hi[j][i]), f[2 * i + 1] - bf16hi_f(hi[j][i]));
           }
-          *reinterpret_cast<uint4*>(ahi + q * 16) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-          *reinterpret_cast<uint4*>(ahi + G.QR * 16 + q * 16) =
-              make_uint4(lo[0], lo[1], lo[2], lo[3]);
-        } else {
-          // Bytes S q .. S q + 15 (S q is a multiple of 4 when S is).
-          const int off = S * q;
-          const uint32_t* w32 = reinterpret_cast<const uint32_t*>(row + (off & ~3));
-          const uint32_t sh = (off & 3) * 8;
-          uint32_t w[5];
+        }
 #pragma unroll
-          for (int j = 0; j < 5; ++j) w[j] = (S % 4 == 0 && j == 4) ? 0u : w32[j];
+        for (int j = 0; j < NG; ++j) {
+          uint32_t h4[4], l4[4];
+#pragma unroll
+          for (int d = 0; d < 8 / S; ++d)
+#pragma unroll
+            for (int i = 0; i < SP; ++i) {
+              if (d == 0) {
+                h4[i] = hi[j][i];
+                l4[i] = lo[j][i];
+              } else {
+                // Lane + d: of this group, or of the next one past lane 31.
+                const int jn = j + 1 < NL ? j + 1 : j;
+                const int from = (lane + d) & 31;
+                h4[d * SP + i] = __shfl_sync(0xffffffffu, lane < d ? hi[jn][i] : hi[j][i], from);
+                l4[d * SP + i] = __shfl_sync(0xffffffffu, lane < d ? lo[jn][i] : lo[j][i], from);
+              }
+            }
+          const int q = lane + 32 * j;
+          if (q < G.QR) {
+            *reinterpret_cast<uint4*>(ahi + q * 16) = make_uint4(h4[0], h4[1], h4[2], h4[3]);
+            *reinterpret_cast<uint4*>(ahi + G.QR * 16 + q * 16) =
+                make_uint4(l4[0], l4[1], l4[2], l4[3]);
+          }
+        }
+      } else {
+        // Bytes S q .. S q + 15 (S q is a multiple of 4 when S is).
+        constexpr int NW = S % 4 == 0 ? 4 : 5;
+        auto get = [&](int q, uint32_t (&w)[NW]) {
+          const uint32_t* w32 = reinterpret_cast<const uint32_t*>(row + ((S * q) & ~3));
+#pragma unroll
+          for (int j = 0; j < NW; ++j) w[j] = w32[j];
+        };
+        auto put = [&](int q, const uint32_t (&w)[NW]) {
+          const uint32_t sh = ((S * q) & 3) * 8;
           uint32_t v[4];
 #pragma unroll
           for (int j = 0; j < 4; ++j)
-            v[j] = S % 4 == 0 ? w[j] : __funnelshift_r(w[j], w[j + 1], sh);
+            v[j] = S % 4 == 0 ? w[j] : __funnelshift_r(w[j], w[(j + 1) % NW], sh);
           *reinterpret_cast<uint4*>(ahi + q * 16) = make_uint4(v[0], v[1], v[2], v[3]);
+        };
+        uint32_t w[kM / 32][NW];
+#pragma unroll
+        for (int j = 0; j < kM / 32; ++j) get(lane + 32 * j, w[j]);
+#pragma unroll
+        for (int j = 0; j < kM / 32; ++j) put(lane + 32 * j, w[j]);
+        for (int q = kM + lane; q < G.QR; q += 32) {
+          get(q, w[0]);
+          put(q, w[0]);
         }
       }
       fence_async_smem();
       __syncwarp();
       if (lane == 0) {
-        mbar_arrive(&ready[i]);
-        mbar_arrive(&raw_free[st]);
+        mbar_arrive(&ready[kb % AB]);
+        if (t + NR < nsteps) load_stage(t + NR);
       }
-      if (++i == G.NA) i = 0;
-      if (++st == kNRaw) { st = 0; rph ^= 1; }
+    }
+    // After a wait that gave up: every load issued lands before the item ends.
+    if (lane == 0) {
+      volatile int no_abort = 0;
+      for (int r = t; r < min(t + NR, nsteps); r += kBuilders)
+        mbar_wait(&raw_full[r % NR], (r / NR) & 1, &no_abort, kSpinLimit);
     }
   } else {
     // ---- Epilogue ---------------------------------------------------------------
-    typedef typename std::conditional<SPLIT, float, int>::type AT;  // running sums
-    const int sp = warp - kBuilders;  // TMEM sub-partition (warp % 4)
-    const int m = sp * 32 + lane;
-    const uint32_t lane_base = tmem_base + (static_cast<uint32_t>(sp * 32) << 16);
-    const uint32_t ring = lane_base + kRingCol;
-    // The item's fields in registers: the item lives in shared memory, and
-    // the score loop would otherwise reload them on every slot.
-    const auto ea_W = a.W;
-    const auto ea_accum = a.accum;
-    const int ea_idx_op = IDX ? a.idx_op : -1;
-    const auto ea_dst = a.dst;
-    const auto ea_dst_f64 = a.dst_f64;
-    const auto ea_dst_pitch = a.dst_pitch;
-    const auto ea_measure = a.measure;
-    const auto ea_nch = a.nch;
-    const auto ea_xs_out = a.xs_out;
-    const auto ea_y0 = a.y0;
-    const auto ea_yend = a.yend;
-    const double etd = cs.et;
-    const float ret = (float)(1.0 / sqrt(etd));  // 1 / sqrt(E_T)
-    // Score of one position from its product sum cv and window energy ev.
-    // Split sources: SqrDistance's terms cancel near a match, so its
-    // numerator is formed in FP64; the _Norm scale of an F32 map is taken in
-    // FP32 (relative error a few 1e-7), of an F64 map in FP64. U8: exact
-    // integers and the plain path's float or double formulas (bit-identical).
-    // Best-match state of this lane (ocipProximityIndx).
-    IdxState ib;
-    ib.v = 0.f;
-    ib.key = 0ull;
-    ib.have = 0;
-    ib.nan = 0;
-    const int idx_ngx = (ea_W + 255) >> 8;
-    auto idx_update = [&](float v, int x, int y) { idx_state_update(ib, v, x, y, ea_idx_op, idx_ngx); };
-    // U8 _Norm: float arithmetic where the plain path's float sums are exact.
-    const bool u8_float = (double)a.tw * a.th * 65025.0 <= 16777216.0;
-    // Scores with the measure fixed at compile time (MT::value), so that the
-    // S positions of a slot are straight-line, independent work.
-    auto num_of = [&](auto mt, AT cv, double ev) -> double {
-      constexpr int M = decltype(mt)::value;
-      const double cc = (double)cv;
-      if (M == kCrossCorr || M == kCrossCorrNorm) return cc;
-      return ev - 2.0 * cc + etd;
-    };
-    auto score_f = [&](auto mt, AT cv, double ev) -> float {
-      constexpr int M = decltype(mt)::value;
-      if (SPLIT) {
-        const double num = num_of(mt, cv, ev);
-        if (M == kCrossCorr || M == kSqrDistance) return (float)num;
-        return (float)num * (rsqrtf((float)ev) * ret);
-      } else {
-        // Exact in int32: each of C, E_S, E_T <= 64 * 64 * 255^2 < 2^28.
-        const int cc = static_cast<int>(cv);
-        const int es = static_cast<int>(ev);
-        const int ei = static_cast<int>(etd);
-        const int num = (M == kCrossCorr || M == kCrossCorrNorm) ? cc : es - 2 * cc + ei;
-        if (M == kCrossCorr || M == kSqrDistance) return __int2float_rn(num);
-        if (u8_float) return __fdiv_rn((float)num, __fsqrt_rn(__fmul_rn((float)es, (float)ei)));
-        return (float)__ddiv_rn((double)num, __dsqrt_rn(__dmul_rn((double)es, (double)ei)));
-      }
-    };
-    auto score_d = [&](auto mt, AT cv, double ev) -> double {
-      constexpr int M = decltype(mt)::value;
-      if (SPLIT) {
-        const double num = num_of(mt, cv, ev);
-        if (M == kCrossCorr || M == kSqrDistance) return num;
-        return num * rsqrt(ev * etd);
-      } else {
-        const int cc = static_cast<int>(cv);
-        const int es = static_cast<int>(ev);
-        const int ei = static_cast<int>(etd);
-        const int num = (M == kCrossCorr || M == kCrossCorrNorm) ? cc : es - 2 * cc + ei;
-        if (M == kCrossCorr || M == kSqrDistance) return (double)num;
-        if (u8_float)
-          return (double)__fdiv_rn((float)num, __fsqrt_rn(__fmul_rn((float)es, (float)ei)));
-        return __ddiv_rn((double)num, __dsqrt_rn(__dmul_rn((double)es, (double)ei)));
-      }
-    };
-    // Row energies of the rows block kk's slots complete (entering: staged
-    // row u; leaving: staged row u - th), S positions of this lane each,
-    // loaded before the block's MMAs are waited for. The window energy of
-    // each position is an FP64 running sum over the slots, in order.
-    typedef typename std::conditional<SPLIT, float, int>::type RT;
-    const int xl = ea_xs_out + S * m;
-    RT rin[BS][S], rout[BS][S];
-    double esum[S];
-#pragma unroll
-    for (int p = 0; p < S; ++p) esum[p] = 0.0;
-#pragma unroll
-    for (int g = 0; g < BS; ++g)
-#pragma unroll
-      for (int p = 0; p < S; ++p) rin[g][p] = rout[g][p] = RT(0);  // CrossCorr: no energies
-    auto load_rows = [&](RT (&v)[S], int sr) {
-      const bool row_ok = need_e && sr >= 0 && sr < a.H;
-      const RT* er = reinterpret_cast<const RT*>(a.energy + (size_t)ch * a.e_plane +
-                                                 (size_t)(row_ok ? sr : 0) * a.e_pitch);
-      if (row_ok && xl + S <= ea_W) {
-        if (S == 2) {
-          const uint2 q = *reinterpret_cast<const uint2*>(er + xl);
-          memcpy(v, &q, sizeof(q));
-        } else {
-#pragma unroll
-          for (int j = 0; j < S / 4; ++j) {
-            const uint4 q = reinterpret_cast<const uint4*>(er + xl)[j];
-            memcpy(&v[4 * j], &q, sizeof(q));
-          }
-        }
-      } else {
-#pragma unroll
-        for (int p = 0; p < S; ++p) v[p] = row_ok && xl + p < ea_W ? er[xl + p] : RT(0);
-      }
-    };
-    auto load_energies = [&](int kk) {
-#pragma unroll
-      for (int g = 0; g < BS; ++g) {
-        const int u = kk * BS + g;
-        const bool in = u < nsteps;
-        load_rows(rin[g], in ? r_begin + u : -1);
-        load_rows(rout[g], in && u >= a.th ? r_begin + u - a.th : -1);
-      }
-    };
-    uint32_t zero[16];
-#pragma unroll
-    for (int j = 0; j < 16; ++j) zero[j] = 0u;
-    for (int c = 0; c < kRingCols; c += 16) tmem_st16(ring + c, zero);
-    tmem_st_wait();
-    for (int k = 0; k * BS < nsteps; ++k) {
-      const int t0 = k * BS;
-      if (need_e) load_energies(k);
-      bool ok = mbar_wait(&blk_full[k & 1], (k >> 1) & 1, abort_flag, kSpinLimit);
-      // tcgen05.ld/st are warp-collective: the whole warp takes one branch.
-      if (!__all_sync(0xffffffffu, ok)) break;
-      tc_fence_after();
-      const uint32_t part = lane_base + (k & 1) * kPartCols;
-      // Relative chunk i of the block lives at ring chunk (k + i) mod NCH.
-      // Chunks 1 .. NCH - 1 hold open slots: ring += partial.
-      for (int c16 = 1; c16 < NCH; ++c16) {
-        const uint32_t rc = ring + 16 * ((k + c16) % NCH);
-        uint32_t vp[16], vr[16];
-        tmem_ld16x(part + 16 * c16, vp);
-        tmem_ld16x(rc, vr);
-        tmem_ld_wait();
-#pragma unroll
-        for (int j = 0; j < 16; ++j) {
-          if (SPLIT)
-            vr[j] = __float_as_uint(__fadd_rn(__uint_as_float(vr[j]), __uint_as_float(vp[j])));
-          else
-            vr[j] += vp[j];  // exact int32 sums
-        }
-        tmem_st16(rc, vr);
-      }
-      // Chunk 0: the BS slots t0 .. t0 + BS - 1 this block completes. Their
-      // ring columns are cleared for the slots NS later.
-      AT val[16];
-      {
-        const uint32_t rc = ring + 16 * (k % NCH);
-        uint32_t vp[16], vr[16];
-        tmem_ld16x(part, vp);
-        tmem_ld16x(rc, vr);
-        tmem_ld_wait();
-#pragma unroll
-        for (int j = 0; j < 16; ++j) {
-          if (SPLIT)
-            val[j] = __fadd_rn(__uint_as_float(vr[j]), __uint_as_float(vp[j]));
-          else
-            val[j] = static_cast<int>(vr[j] + vp[j]);
-        }
-        tmem_st16(rc, zero);
-      }
-      tmem_st_wait();
-      // The partial has been read: the MMAs may refill it (block k + 2).
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&buf_free[k & 1]);
-      // The block's completed slots: window energies (running sums, in
-      // order), scores and stores, specialised per measure.
-      auto slots = [&](auto mt) {
-#pragma unroll
-        for (int g = 0; g < BS; ++g) {
-          const int u = t0 + g;
-          const int yd = ea_y0 + u - R + 1;
-          if (u >= nsteps) break;
-          double e[S];
-#pragma unroll
-          for (int p = 0; p < S; ++p) {
-            esum[p] += static_cast<double>(rin[g][p]) - static_cast<double>(rout[g][p]);
-            e[p] = esum[p];
-          }
-          if (u >= R - 1 && yd < ea_yend) {
-            char* orow = ea_dst + (size_t)yd * ea_dst_pitch;
-            const int x0 = xl;
-            if (ea_nch == 1 && !ea_dst_f64 && x0 + S <= ea_W) {
-              float outf[S];
-#pragma unroll
-              for (int p = 0; p < S; ++p) outf[p] = score_f(mt, val[g * S + p], e[p]);
-              if (IDX && ea_idx_op >= 0) {
-#pragma unroll
-                for (int p = 0; p < S; ++p) idx_update(outf[p], x0 + p, yd);
-              }
-              if (ea_dst != nullptr) {
-                float* o = reinterpret_cast<float*>(orow) + x0;
-                if (S % 4 == 0) {
-#pragma unroll
-                  for (int j = 0; j < S / 4; ++j)
-                    reinterpret_cast<float4*>(o)[j] = make_float4(
-                        outf[(4 * j) % S], outf[(4 * j + 1) % S], outf[(4 * j + 2) % S],
-                        outf[(4 * j + 3) % S]);
-                } else {
-#pragma unroll
-                  for (int j = 0; j < S / 2; ++j)
-                    reinterpret_cast<float2*>(o)[j] =
-                        make_float2(outf[(2 * j) % S], outf[(2 * j + 1) % S]);
-                }
-              }
-            } else {
-#pragma unroll
-              for (int p = 0; p < S; ++p) {
-                const int x = x0 + p;
-                if (x >= ea_W) break;
-                const size_t xo = (size_t)x * ea_nch + ch;
-                if (ea_dst_f64 && ea_accum) {
-                  reinterpret_cast<double*>(orow)[xo] += score_d(mt, val[g * S + p], e[p]);
-                } else if (ea_dst_f64) {
-                  reinterpret_cast<double*>(orow)[xo] = score_d(mt, val[g * S + p], e[p]);
-                } else {
-                  const float v = score_f(mt, val[g * S + p], e[p]);
-                  if (IDX && ea_idx_op >= 0) idx_update(v, x, yd);
-                  if (ea_dst != nullptr) reinterpret_cast<float*>(orow)[xo] = v;
-                }
-              }
-            }
-          }
-        }
-      };
-      switch (ea_measure) {
-        case kSqrDistance: slots(std::integral_constant<int, kSqrDistance>()); break;
-        case kSqrDistanceNorm: slots(std::integral_constant<int, kSqrDistanceNorm>()); break;
-        case kCrossCorrNorm: slots(std::integral_constant<int, kCrossCorrNorm>()); break;
-        default: slots(std::integral_constant<int, kCrossCorr>()); break;
-      }
-      if (!__all_sync(0xffffffffu, ok)) break;
-    }
-    if (IDX && ea_idx_op >= 0) {
-      // The warp's best: same rule, then lane 0 writes the warp's record.
-      const bool is_min = ea_idx_op == 0 || ea_idx_op == 2;
-#pragma unroll
-      for (int d = 16; d > 0; d >>= 1) {
-        const float ov = __shfl_xor_sync(0xffffffffu, ib.v, d);
-        const unsigned long long ok2 = __shfl_xor_sync(0xffffffffu, ib.key, d);
-        const int oh = __shfl_xor_sync(0xffffffffu, ib.have, d);
-        ib.nan |= __shfl_xor_sync(0xffffffffu, ib.nan, d);
-        const bool take = oh && (!ib.have || (is_min ? ov < ib.v : ov > ib.v) ||
-                                 (ov == ib.v && ok2 < ib.key));
-        if (take) {
-          ib.v = ov;
-          ib.key = ok2;
-          ib.have = 1;
-        }
-      }
-      if (lane == 0) {
-        const int item = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
-        IdxRecord r;
-        r.v = ib.v;
-        r.have = ib.have;
-        r.key = ib.key;
-        r.nan = ib.nan;
-        r.pad = 0;
-        reinterpret_cast<IdxRecord*>(a.idx_out)[item * kEpilogue + sp] = r;
-      }
+    const uint32_t tm = tmem_base;
+    switch (a.measure) {
+      case kSqrDistance:
+        run_epilogue<ELEM, S, IDX, kSqrDistance>(a, cs, tm, blk_full, buf_free, r_begin, nsteps);
+        break;
+      case kSqrDistanceNorm:
+        run_epilogue<ELEM, S, IDX, kSqrDistanceNorm>(a, cs, tm, blk_full, buf_free, r_begin,
+                                                     nsteps);
+        break;
+      case kCrossCorrNorm:
+        run_epilogue<ELEM, S, IDX, kCrossCorrNorm>(a, cs, tm, blk_full, buf_free, r_begin, nsteps);
+        break;
+      default:
+        run_epilogue<ELEM, S, IDX, kCrossCorr>(a, cs, tm, blk_full, buf_free, r_begin, nsteps);
+        break;
     }
   }
 
@@ -886,11 +1129,11 @@ __device__ __forceinline__ void run_item(const ItemArgs& a, unsigned char* smem,
   __syncthreads();
   tc_fence_after();
   if (threadIdx.x == 0) {
-    for (int i = 0; i < kNRaw; ++i) {
-      mbar_inval(&raw_full[i]);
-      mbar_inval(&raw_free[i]);
+    for (int i = 0; i < NR; ++i) mbar_inval(&raw_full[i]);
+    for (int i = 0; i < AB; ++i) {
+      mbar_inval(&ready[i]);
+      mbar_inval(&a_free[i]);
     }
-    for (int i = 0; i < G.NA; ++i) mbar_inval(&ready[i]);
     for (int i = 0; i < 2; ++i) {
       mbar_inval(&blk_full[i]);
       mbar_inval(&buf_free[i]);
