@@ -23,8 +23,7 @@ NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 COMMON = ["-std=c++17", "-O3", "-lineinfo", "-Xcompiler", "-fPIC,-fvisibility=hidden",
           "-I", os.path.join(ROOT, "include"), "-I", CSRC]
-# The kernels of a file are optimised in parallel (a full build takes minutes otherwise).
-CU_FLAGS = ARCH + COMMON + ["-Xptxas", "-O3", "--expt-relaxed-constexpr", "--split-compile=0"]
+CU_FLAGS = ARCH + COMMON + ["-Xptxas", "-O3", "--expt-relaxed-constexpr"]
 
 
 def sources():

@@ -48,7 +48,7 @@ struct DevImage {
 // tt_scratch: 64 bytes of device memory for the per-channel template energy.
 cudaError_t launch_proximity_plain(Measure m, const DevImage& src,
                                    const DevImage& tmpl, const DevImage& dst,
-                                   void* tt_scratch, cudaStream_t stream);
+                                   void* tt_scratch, int sm_count, cudaStream_t stream);
 
 // AbsDistance of a U8 or S8 source with packed-byte SAD (four taps per
 // instruction, exact uint32 sums); launch_proximity_plain routes 8-bit

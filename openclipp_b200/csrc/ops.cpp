@@ -100,7 +100,7 @@ void proximity_run(Context& ctx, Measure m, Image& S, Image& T, Image& D, int pa
   }
   if (!done) {
     void* tt = ctx.scratch(Context::kTemplateEnergy, 64);
-    e = launch_proximity_plain(m, s, t, d, tt, ctx.stream);
+    e = launch_proximity_plain(m, s, t, d, tt, ctx.sm_count, ctx.stream);
     ctx.last_path = OCIP_PATH_PLAIN;
   }
   check_cuda(e, "proximity kernel launch");
@@ -418,7 +418,7 @@ void proximity_index(int measure, int op, ocipImage hs, ocipImage ht, ocipImage 
       ctx.last_path = OCIP_PATH_TENSOR;
     } else {
       void* tt = ctx.scratch(Context::kTemplateEnergy, 64);
-      e = launch_proximity_plain(m, s, t, map, tt, ctx.stream);
+      e = launch_proximity_plain(m, s, t, map, tt, ctx.sm_count, ctx.stream);
       ctx.last_path = OCIP_PATH_PLAIN;
     }
     check_cuda(e, "proximity kernel launch");

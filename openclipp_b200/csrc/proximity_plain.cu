@@ -15,15 +15,16 @@
 // 2^24 (then identical to the reference), in double otherwise (exact while
 // sums stay below 2^53, i.e. for every 8/16-bit case of practical size).
 //
-// Tiling. A CTA of 8 warps owns a 256 x (8*RY) output tile: lane l owns RX=8
-// consecutive columns, warp w owns RY consecutive rows. Source rows of the
-// tile (plus halo, converted to the compute type) and template rows sit in
-// shared memory. For each source row q, a warp slides an RX+8 wide register
-// window along x and applies it to all of its RY output rows at once, each
-// with its own template row h = q - j, which keeps per-output order h-major.
-// Shared-memory rows are stored in 16-byte chunks with one pad chunk after
-// every 8, so the lanes' stride-2 (float) or stride-4 (double) chunk accesses
-// hit distinct banks. Very tall templates are processed in row bands.
+// Tiling. A CTA of NW warps owns a 32 RX x (NW RY) output tile: lane l owns RX
+// consecutive columns, warp w owns RY consecutive rows (launch_typed chooses the
+// tile). Source rows of the tile (plus halo, converted to the compute type) and
+// template rows sit in shared memory. For each source row q, a warp slides an
+// RX+8 wide register window along x and applies it to all of its RY output rows
+// at once, each with its own template row h = q - j, which keeps per-output
+// order h-major. Shared-memory rows are stored in 16-byte chunks; where a lane
+// owns more than one chunk, one pad chunk after every 8 makes the lanes'
+// stride-2 or stride-4 chunk accesses hit distinct banks. Very tall templates
+// are processed in row bands.
 //
 // FP32 compute types run on sm_100's packed FP32 arithmetic over pairs of
 // output rows (PackedRows below), specialised on the width of the template's
@@ -37,10 +38,6 @@
 namespace ocipb {
 namespace {
 
-constexpr int kThreads = 256;
-constexpr int kWarps = kThreads / 32;
-constexpr int RX = 8;     // outputs per thread along x
-constexpr int TX = 32 * RX;
 constexpr int WCH = 8;    // template columns per inner step
 constexpr int kSmemBudget = 200 * 1024;
 
@@ -64,6 +61,8 @@ struct PlainParams {
   const void* tt;  // per-channel template energy (compute type), _Norm only
   int dst_f64;
   int W, H, nch, dst_nch;
+  int type;  // source type of the packed form: U8, S8 or F32
+  int nx;    // tiles along x (all tiles in grid dimension x: any height fits)
   int tw, th, twp;
   int rowBytes;     // bytes per shared-memory source row (with pad chunks)
   int RB;           // source rows per band
@@ -84,20 +83,27 @@ __device__ __forceinline__ double dv(double a, double b) { return __ddiv_rn(a, b
 __device__ __forceinline__ float sq(float a) { return __fsqrt_rn(a); }
 __device__ __forceinline__ double sq(double a) { return __dsqrt_rn(a); }
 
+// Rows of RX elements a lane: with one 16-byte chunk a lane (FP32, RX = 4) the
+// lanes' chunks are adjacent and need no padding.
+template <typename CT>
+__host__ __device__ constexpr bool padded(int RX) {
+  return RX * (int)sizeof(CT) > 16;
+}
+
 // Byte offset of logical element e of a shared-memory row: 16-byte chunks,
 // one pad chunk after every 8 chunks.
-template <typename CT>
+template <typename CT, int RX>
 __device__ __forceinline__ int phys_off(int e) {
   constexpr int E = 16 / sizeof(CT);
   const int c = e / E;
-  return (c + (c >> 3)) * 16 + (e % E) * (int)sizeof(CT);
+  return (padded<CT>(RX) ? c + (c >> 3) : c) * 16 + (e % E) * (int)sizeof(CT);
 }
 
-template <typename CT>
+template <typename CT, int RX>
 __host__ __device__ inline int row_bytes_for(int L) {
   const int E = 16 / (int)sizeof(CT);
   const int chunks = (L + E - 1) / E;
-  return (chunks + chunks / 8 + 1) * 16;
+  return (chunks + (padded<CT>(RX) ? chunks / 8 : 0) + 1) * 16;
 }
 
 // Packed FP32 form (every measure, FP32 compute type). Output rows 2jp and
@@ -125,7 +131,7 @@ struct PackedRows {
 // One chunk of KMAX template columns for a pair of output rows whose template
 // rows both lie inside the template: sd[e] holds window element e in both
 // halves, tp[k] the pair's (possibly negated) template values of column k.
-template <int MEAS, int KMAX>
+template <int MEAS, int KMAX, int RX>
 __device__ __forceinline__ void pair_chunk(float2 (&acc)[RX], float2 (&acc2)[RX],
                                            const float2 (&sd)[RX + WCH], const float2 (&tp)[WCH]) {
 #pragma unroll
@@ -150,7 +156,7 @@ __device__ __forceinline__ void pair_chunk(float2 (&acc)[RX], float2 (&acc2)[RX]
 
 // The same for one row of the pair (H = 0: row 2jp, the .x halves; H = 1: row
 // 2jp + 1, the .y halves) when the other row's template row lies outside.
-template <int MEAS, int KMAX, int H>
+template <int MEAS, int KMAX, int H, int RX>
 __device__ __forceinline__ void half_chunk(float2 (&acc)[RX], float2 (&acc2)[RX],
                                            const float (&win)[RX + WCH], const float (&tv)[WCH]) {
 #pragma unroll
@@ -175,7 +181,7 @@ __device__ __forceinline__ void half_chunk(float2 (&acc)[RX], float2 (&acc2)[RX]
 }
 
 // One template-column chunk applied to one output row.
-template <typename CT, int MEAS>
+template <typename CT, int MEAS, int RX>
 __device__ __forceinline__ void apply_chunk(CT (&acc)[RX], CT (&acc2)[RX],
                                             const CT (&win)[RX + WCH],
                                             const CT (&tv)[WCH], int kmax) {
@@ -206,12 +212,15 @@ __device__ __forceinline__ void apply_chunk(CT (&acc)[RX], CT (&acc2)[RX],
   }
 }
 
+// NW warps of RY output rows each. TYPE: the source type, or -1 for p.type.
 // KT: for the packed FP32 form, the columns of the template's last chunk,
 // tw - WCH * ((tw - 1) / WCH), in 1 .. WCH; 0 for the other forms.
-template <int TYPE, typename CT, int MEAS, int RY, int KT>
-__global__ void __launch_bounds__(kThreads, sizeof(CT) == 4 ? 2 : 1)
+template <int TYPE, typename CT, int MEAS, int RX, int RY, int NW, int KT>
+__global__ void __launch_bounds__(NW * 32, sizeof(CT) == 4 ? 16 / NW : 1)
     prox_plain_kernel(const PlainParams p) {
-  using ET = typename ElemOf<TYPE>::T;
+  constexpr int kThreads = NW * 32;
+  constexpr int TX = 32 * RX;
+  constexpr int kWarps = NW;
   constexpr bool kNorm = (MEAS == kCrossCorrNorm || MEAS == kSqrDistanceNorm);
   constexpr bool kPacked = PackedRows<CT, MEAS>::value;
   constexpr int TY = kWarps * RY;
@@ -222,8 +231,8 @@ __global__ void __launch_bounds__(kThreads, sizeof(CT) == 4 ? 2 : 1)
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
   const int c = blockIdx.z;
-  const int x0 = blockIdx.x * TX;
-  const int y0 = blockIdx.y * TY;
+  const int x0 = (blockIdx.x % p.nx) * TX;
+  const int y0 = (blockIdx.x / p.nx) * TY;
   const int left = -(p.tw / 2);
   const int top = -(p.th / 2);
   const int L = TX + p.twp;          // logical elements per source row
@@ -234,9 +243,9 @@ __global__ void __launch_bounds__(kThreads, sizeof(CT) == 4 ? 2 : 1)
   CT acc[RY][RX];
   CT acc2[RY][RX];
   // Packed form: output rows (2jp, 2jp + 1) of column i.
-  float2 accr[RY / 2][RX], accr2[RY / 2][RX];
+  float2 accr[(RY + 1) / 2][RX], accr2[(RY + 1) / 2][RX];
 #pragma unroll
-  for (int j = 0; j < RY / 2; ++j)
+  for (int j = 0; j < (RY + 1) / 2; ++j)
 #pragma unroll
     for (int i = 0; i < RX; ++i) {
       accr[j][i] = make_float2(0.f, 0.f);
@@ -261,56 +270,69 @@ __global__ void __launch_bounds__(kThreads, sizeof(CT) == 4 ? 2 : 1)
     // lanes along the row (coalesced), zero outside the image. Sources of the
     // compute type are copied asynchronously (no register round trip), the
     // copies overlapping the template staging below.
-    for (int qq = warp; qq < g1 - g0; qq += kWarps) {
-      const int gy = y0 + top + g0 + qq;
-      const bool row_in = gy >= 0 && gy < p.H;
-      const ET* grow =
-          reinterpret_cast<const ET*>(p.src + (size_t)(row_in ? gy : 0) * p.src_pitch) + c;
-      unsigned char* srow = s_src + (size_t)qq * p.rowBytes;
-      if constexpr (std::is_same<CT, ET>::value) {
-        // Asynchronous copies, zero-filled outside the image (source size 0).
-#pragma unroll 4
-        for (int e = lane; e < L; e += 32) {
-          const int gx = x0 + left + e;
-          const bool in = row_in && gx >= 0 && gx < p.W;
-          const ET* g = grow + (size_t)(in ? gx : 0) * p.nch;
-          const unsigned sa = (unsigned)__cvta_generic_to_shared(srow + phys_off<CT>(e));
-          asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;\n" ::"r"(sa), "l"(g),
-                       "n"((int)sizeof(ET)), "r"(in ? (int)sizeof(ET) : 0)
-                       : "memory");
-        }
-      } else {
-#pragma unroll 4
-        for (int e = lane; e < L; e += 32) {
-          const int gx = x0 + left + e;
-          CT v = CT(0);
-          if (row_in && gx >= 0 && gx < p.W) v = (CT)grow[(size_t)gx * p.nch];
-          *reinterpret_cast<CT*>(srow + phys_off<CT>(e)) = v;
-        }
-      }
-    }
-    if constexpr (std::is_same<CT, ET>::value) asm volatile("cp.async.commit_group;\n" ::: "memory");
-    // Stage template rows [tg0, tg1), zero-padded to twp columns. The packed
+    //
+    // Then template rows [tg0, tg1), zero-padded to twp columns. The packed
     // form stores row h as the pairs (t(h, w), t(h - 1, w)), negated for the
-    // measures that take differences.
-    // Read-only loads, unrolled, so that a thread's loads are in flight together.
-    const int ntel = (tg1 - tg0) * tstride;
-#pragma unroll 8
-    for (int idx = threadIdx.x; idx < ntel; idx += kThreads) {
-      const int hh = idx / tstride;
-      int w = idx - hh * tstride;
-      int trow = tg0 + hh;
-      if (kPacked) {  // pairs (row h, row h - 1) of column w
-        w = (idx - hh * tstride) >> 1;
-        trow -= (idx - hh * tstride) & 1;
+    // measures that take differences. Read-only loads, unrolled, so that a
+    // thread's loads are in flight together.
+    auto stage = [&](auto type) {
+      using ET = typename ElemOf<decltype(type)::value>::T;
+      for (int qq = warp; qq < g1 - g0; qq += kWarps) {
+        const int gy = y0 + top + g0 + qq;
+        const bool row_in = gy >= 0 && gy < p.H;
+        const ET* grow =
+            reinterpret_cast<const ET*>(p.src + (size_t)(row_in ? gy : 0) * p.src_pitch) + c;
+        unsigned char* srow = s_src + (size_t)qq * p.rowBytes;
+        if constexpr (std::is_same<CT, ET>::value) {
+          // Asynchronous copies, zero-filled outside the image (source size 0).
+#pragma unroll 4
+          for (int e = lane; e < L; e += 32) {
+            const int gx = x0 + left + e;
+            const bool in = row_in && gx >= 0 && gx < p.W;
+            const ET* g = grow + (size_t)(in ? gx : 0) * p.nch;
+            const unsigned sa = (unsigned)__cvta_generic_to_shared(srow + phys_off<CT, RX>(e));
+            asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;\n" ::"r"(sa), "l"(g),
+                         "n"((int)sizeof(ET)), "r"(in ? (int)sizeof(ET) : 0)
+                         : "memory");
+          }
+        } else {
+#pragma unroll 4
+          for (int e = lane; e < L; e += 32) {
+            const int gx = x0 + left + e;
+            CT v = CT(0);
+            if (row_in && gx >= 0 && gx < p.W) v = (CT)grow[(size_t)gx * p.nch];
+            *reinterpret_cast<CT*>(srow + phys_off<CT, RX>(e)) = v;
+          }
+        }
       }
-      CT v = CT(0);
-      if (w < p.tw && trow >= 0)
-        v = (CT)__ldg(reinterpret_cast<const ET*>(
-            p.tmpl + (size_t)trow * p.tmpl_pitch + ((size_t)w * p.nch + c) * sizeof(ET)));
-      s_t[idx] = (kPacked && PackedRows<CT, MEAS>::neg) ? -v : v;
+      const int ntel = (tg1 - tg0) * tstride;
+#pragma unroll 8
+      for (int idx = threadIdx.x; idx < ntel; idx += kThreads) {
+        const int hh = idx / tstride;
+        int w = idx - hh * tstride;
+        int trow = tg0 + hh;
+        if (kPacked) {  // pairs (row h, row h - 1) of column w
+          w = (idx - hh * tstride) >> 1;
+          trow -= (idx - hh * tstride) & 1;
+        }
+        CT v = CT(0);
+        if (w < p.tw && trow >= 0)
+          v = (CT)__ldg(reinterpret_cast<const ET*>(
+              p.tmpl + (size_t)trow * p.tmpl_pitch + ((size_t)w * p.nch + c) * sizeof(ET)));
+        s_t[idx] = (kPacked && PackedRows<CT, MEAS>::neg) ? -v : v;
+      }
+    };
+    if constexpr (TYPE >= 0) {
+      stage(std::integral_constant<int, TYPE>());
+    } else {
+      if (p.type == F32)
+        stage(std::integral_constant<int, F32>());
+      else if (p.type == U8)
+        stage(std::integral_constant<int, U8>());
+      else
+        stage(std::integral_constant<int, S8>());
     }
-    if constexpr (std::is_same<CT, ET>::value) asm volatile("cp.async.wait_all;\n" ::: "memory");
+    asm volatile("cp.async.wait_all;\n" ::: "memory");
     __syncthreads();
 
     // Window of source row q for template columns wc*WCH ..: RX + WCH elements.
@@ -321,13 +343,13 @@ __global__ void __launch_bounds__(kThreads, sizeof(CT) == 4 ? 2 : 1)
       for (int v = 0; v < (RX + WCH) / E; ++v) {
         const int e = e0 + v * E;
         if (sizeof(CT) == 4) {
-          const float4 f = *reinterpret_cast<const float4*>(srow + phys_off<CT>(e));
+          const float4 f = *reinterpret_cast<const float4*>(srow + phys_off<CT, RX>(e));
           win[v * 4 + 0] = (CT)f.x;
           win[v * 4 + 1] = (CT)f.y;
           win[v * 4 + 2] = (CT)f.z;
           win[v * 4 + 3] = (CT)f.w;
         } else {
-          const double2 d = *reinterpret_cast<const double2*>(srow + phys_off<CT>(e));
+          const double2 d = *reinterpret_cast<const double2*>(srow + phys_off<CT, RX>(e));
           win[v * 2 + 0] = (CT)d.x;
           win[v * 2 + 1] = (CT)d.y;
         }
@@ -371,9 +393,9 @@ __global__ void __launch_bounds__(kThreads, sizeof(CT) == 4 ? 2 : 1)
           CT tv[WCH];
           load_tmpl(s_t + (size_t)(h - tg0) * tstride + wc * WCH, tv);
           if (kmax == WCH)
-            apply_chunk<CT, MEAS>(acc[j], acc2[j], win, tv, WCH);
+            apply_chunk<CT, MEAS, RX>(acc[j], acc2[j], win, tv, WCH);
           else
-            apply_chunk<CT, MEAS>(acc[j], acc2[j], win, tv, kmax);
+            apply_chunk<CT, MEAS, RX>(acc[j], acc2[j], win, tv, kmax);
         }
       }
     };
@@ -412,7 +434,7 @@ __global__ void __launch_bounds__(kThreads, sizeof(CT) == 4 ? 2 : 1)
                   tp[2 * m] = make_float2(f.x, f.y);
                   tp[2 * m + 1] = make_float2(f.z, f.w);
                 }
-                pair_chunk<MEAS, KMAX>(accr[jp], accr2[jp], sd, tp);
+                pair_chunk<MEAS, KMAX, RX>(accr[jp], accr2[jp], sd, tp);
               } else if (both != 0) {
                 // The one template row inside: h (output row 2jp) or h - 1
                 // (row 2jp + 1), read from its own staged row.
@@ -426,9 +448,9 @@ __global__ void __launch_bounds__(kThreads, sizeof(CT) == 4 ? 2 : 1)
                   tv[2 * m + 1] = f.z;
                 }
                 if (both == 1)
-                  half_chunk<MEAS, KMAX, 0>(accr[jp], accr2[jp], win, tv);
+                  half_chunk<MEAS, KMAX, 0, RX>(accr[jp], accr2[jp], win, tv);
                 else
-                  half_chunk<MEAS, KMAX, 1>(accr[jp], accr2[jp], win, tv);
+                  half_chunk<MEAS, KMAX, 1, RX>(accr[jp], accr2[jp], win, tv);
               }
             }
           };
@@ -447,8 +469,13 @@ __global__ void __launch_bounds__(kThreads, sizeof(CT) == 4 ? 2 : 1)
   }
 
   // Epilogue: value = sum (or sum / sqrt(sumSS * sumTT)), stored as F32/F64.
+  // The template energy comes from the kernel before, which this one overlaps
+  // up to here.
   CT tt = CT(0);
-  if (kNorm) tt = reinterpret_cast<const CT*>(p.tt)[c];
+  if (kNorm) {
+    cudaGridDependencySynchronize();
+    tt = reinterpret_cast<const CT*>(p.tt)[c];
+  }
 #pragma unroll
   for (int j = 0; j < RY; ++j) {
     const int y = y0 + warp * RY + j;
@@ -495,6 +522,7 @@ template <int TYPE, typename CT>
 __global__ void __launch_bounds__(256) template_energy_kernel(const char* tmpl, size_t pitch,
                                                               int nch, int tw, int th, CT* out) {
   using ET = typename ElemOf<TYPE>::T;
+  cudaTriggerProgrammaticLaunchCompletion();  // the measure's kernel may start
   constexpr int kMaxStage = 32768 / (int)sizeof(CT);
   __shared__ CT st[kMaxStage];
   const int c = blockIdx.x;
@@ -517,11 +545,15 @@ __global__ void __launch_bounds__(256) template_energy_kernel(const char* tmpl, 
   if (threadIdx.x == 0) out[c] = s;
 }
 
-template <int TYPE, typename CT, int MEAS>
-cudaError_t launch_typed(const DevImage& src, const DevImage& tmpl,
-                         const DevImage& dst, void* tt_buf, cudaStream_t st) {
-  constexpr int RY = sizeof(CT) == 4 ? 4 : 2;
-  constexpr int TY = kWarps * RY;
+// NW warps of RY rows a CTA: the launch of one measure.
+template <int TYPE, typename CT, int MEAS, int RX, int RY, int NW>
+cudaError_t launch_tiled(const DevImage& src, const DevImage& tmpl, const DevImage& dst,
+                         void* tt_buf, cudaStream_t st) {
+  constexpr bool kPacked = PackedRows<CT, MEAS>::value;
+  // One packed kernel for all its source types; F32 on the large tile, which the
+  // largest images take, has a kernel without the others' staging code.
+  constexpr int KTYPE = kPacked && (TYPE != F32 || RX * RY < 32) ? -1 : TYPE;
+  constexpr int TX = 32 * RX, TY = NW * RY;
   PlainParams p;
   p.src = (const char*)src.ptr;
   p.src_pitch = src.pitch;
@@ -534,19 +566,20 @@ cudaError_t launch_typed(const DevImage& src, const DevImage& tmpl,
   p.H = src.height;
   p.nch = src.nch;
   p.dst_nch = dst.nch;
+  p.type = TYPE;
+  p.nx = (src.width + TX - 1) / TX;
   p.tw = tmpl.width;
   p.th = tmpl.height;
   p.twp = (p.tw + WCH - 1) / WCH * WCH;
   p.tt = tt_buf;
   const int L = TX + p.twp;
-  p.rowBytes = row_bytes_for<CT>(L);
+  p.rowBytes = row_bytes_for<CT, RX>(L);
   const int qtot = TY + p.th - 1;
   // Band size: all rows if they fit, else as many as the budget allows.
   int RB = qtot;
   auto bytes_for = [&](int rb) {
     const int tb = std::min(p.th, rb + TY - 1);
-    return (size_t)rb * p.rowBytes +
-           (size_t)tb * p.twp * sizeof(CT) * (PackedRows<CT, MEAS>::value ? 2 : 1);
+    return (size_t)rb * p.rowBytes + (size_t)tb * p.twp * sizeof(CT) * (kPacked ? 2 : 1);
   };
   while (RB > 1 && bytes_for(RB) > (size_t)kSmemBudget) RB = (RB + 1) / 2;
   if (bytes_for(RB) > (size_t)kSmemBudget) return cudaErrorInvalidValue;
@@ -561,37 +594,88 @@ cudaError_t launch_typed(const DevImage& src, const DevImage& tmpl,
         (const char*)tmpl.ptr, tmpl.pitch, tmpl.nch, p.tw, p.th, (CT*)tt_buf);
     count_launches(1);
   }
-  auto kern = prox_plain_kernel<TYPE, CT, MEAS, RY, PackedRows<CT, MEAS>::value ? WCH : 0>;
-  if constexpr (PackedRows<CT, MEAS>::value) {
+  auto kern = prox_plain_kernel<KTYPE, CT, MEAS, RX, RY, NW, kPacked ? WCH : 0>;
+  if constexpr (kPacked) {
     switch (p.tw - WCH * ((p.tw - 1) / WCH)) {
-      case 1: kern = prox_plain_kernel<TYPE, CT, MEAS, RY, 1>; break;
-      case 2: kern = prox_plain_kernel<TYPE, CT, MEAS, RY, 2>; break;
-      case 3: kern = prox_plain_kernel<TYPE, CT, MEAS, RY, 3>; break;
-      case 4: kern = prox_plain_kernel<TYPE, CT, MEAS, RY, 4>; break;
-      case 5: kern = prox_plain_kernel<TYPE, CT, MEAS, RY, 5>; break;
-      case 6: kern = prox_plain_kernel<TYPE, CT, MEAS, RY, 6>; break;
-      case 7: kern = prox_plain_kernel<TYPE, CT, MEAS, RY, 7>; break;
-      default: kern = prox_plain_kernel<TYPE, CT, MEAS, RY, 8>; break;
+      case 1: kern = prox_plain_kernel<KTYPE, CT, MEAS, RX, RY, NW, 1>; break;
+      case 2: kern = prox_plain_kernel<KTYPE, CT, MEAS, RX, RY, NW, 2>; break;
+      case 3: kern = prox_plain_kernel<KTYPE, CT, MEAS, RX, RY, NW, 3>; break;
+      case 4: kern = prox_plain_kernel<KTYPE, CT, MEAS, RX, RY, NW, 4>; break;
+      case 5: kern = prox_plain_kernel<KTYPE, CT, MEAS, RX, RY, NW, 5>; break;
+      case 6: kern = prox_plain_kernel<KTYPE, CT, MEAS, RX, RY, NW, 6>; break;
+      case 7: kern = prox_plain_kernel<KTYPE, CT, MEAS, RX, RY, NW, 7>; break;
+      default: kern = prox_plain_kernel<KTYPE, CT, MEAS, RX, RY, NW, 8>; break;
     }
   }
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)smem);
   if (e != cudaSuccess) return e;
-  dim3 grid((p.W + TX - 1) / TX, (p.H + TY - 1) / TY, src.nch);
-  kern<<<grid, kThreads, smem, st>>>(p);
+  // With a template energy kernel before it, the measure's kernel starts while
+  // that one runs (a serial chain of th tw additions on one SM: 4 us for 16 x
+  // 16, 9 us for 31 x 31) and waits for it before the scores.
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)p.nx * ((p.H + TY - 1) / TY), 1, src.nch);
+  cfg.blockDim = dim3(NW * 32);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr = {};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = kNorm ? 1 : 0;
+  e = cudaLaunchKernelEx(&cfg, kern, p);
   count_launches(1);
-  return cudaGetLastError();
+  return e != cudaSuccess ? e : cudaGetLastError();
+}
+
+// Tile of a CTA. Packed FP32 form: 256 x 32 outputs (8 warps of 8 x 4 a
+// thread) reuse each window register and staged row most, but a small image
+// has fewer such tiles than the chip has SMs (512 x 512: 32), so 128 x 16 (8
+// warps of 4 x 2) and 128 x 8 (4 warps) serve those. The busiest SM computes
+// ceil(tiles / SMs) tiles; the tile with the least outputs there is taken, each
+// weighted by its time per output on a full chip (31 x 31: 128 x 16 took 1.13
+// (AbsDistance) to 1.27 (CrossCorr) of 256 x 32, 128 x 8 1.17 to 1.33, more
+// with few tiles), and an SM with one 8-warp tile alone 1.15 longer than its
+// share of two. Measured, us: 512 x 512 U8 16 x 16 CrossCorr_Norm 37.2 (256 x
+// 32), 14.8 (128 x 16), 18.3 (128 x 8); 1021 x 767 F32 31 x 31 SqrDistance_Norm
+// 119, 94.5, 98.7; 256 x 300 F32 64 x 64 CrossCorr_Norm 323, 99, 72; 1024 x 1024
+// F32 31 x 31 AbsDistance 82.3, 89.0, 84.1; 2048 x 2048 F32 31 x 31 CrossCorr 187,
+// 209, 218.
+//
+// FP64: 256 x 8 (8 warps of 8 x 1): half the accumulators of 8 x 2, so that two
+// CTAs share an SM. 512 x 512 U16 31 x 31 CrossCorr 68.0 -> 43.4 us, 1500 x 1300
+// U8 31 x 31 CrossCorr 262 -> 222, 1920 x 1080 U16 31 x 31 SqrDistance 349 -> 335
+// (640 x 480 U8 31 x 31 SqrDistance_Norm 127 -> 139: 180 tiles, two rounds).
+template <int TYPE, typename CT, int MEAS>
+cudaError_t launch_typed(const DevImage& src, const DevImage& tmpl,
+                         const DevImage& dst, void* tt_buf, int sm_count, cudaStream_t st) {
+  if constexpr (PackedRows<CT, MEAS>::value) {
+    auto cost = [&](int tx, int ty, double weight, double alone) {
+      const long long tiles = (long long)((src.width + tx - 1) / tx) *
+                              ((src.height + ty - 1) / ty) * src.nch;
+      const long long most = (tiles + sm_count - 1) / sm_count;
+      return (double)most * tx * ty * weight * (most == 1 ? alone : 1.0);
+    };
+    const double large = cost(256, 32, 1.0, 1.15), mid = cost(128, 16, 1.25, 1.15),
+                 small = cost(128, 8, 1.45, 1.0);
+    if (small < mid && small < large)
+      return launch_tiled<TYPE, CT, MEAS, 4, 2, 4>(src, tmpl, dst, tt_buf, st);
+    if (mid < large) return launch_tiled<TYPE, CT, MEAS, 4, 2, 8>(src, tmpl, dst, tt_buf, st);
+    return launch_tiled<TYPE, CT, MEAS, 8, 4, 8>(src, tmpl, dst, tt_buf, st);
+  } else {
+    return launch_tiled<TYPE, CT, MEAS, 8, 1, 8>(src, tmpl, dst, tt_buf, st);
+  }
 }
 
 template <int TYPE, typename CT>
 cudaError_t launch_measure(Measure m, const DevImage& src, const DevImage& tmpl,
-                           const DevImage& dst, void* tt, cudaStream_t st) {
+                           const DevImage& dst, void* tt, int sms, cudaStream_t st) {
   switch (m) {
-    case kSqrDistance: return launch_typed<TYPE, CT, kSqrDistance>(src, tmpl, dst, tt, st);
-    case kSqrDistanceNorm: return launch_typed<TYPE, CT, kSqrDistanceNorm>(src, tmpl, dst, tt, st);
-    case kAbsDistance: return launch_typed<TYPE, CT, kAbsDistance>(src, tmpl, dst, tt, st);
-    case kCrossCorr: return launch_typed<TYPE, CT, kCrossCorr>(src, tmpl, dst, tt, st);
-    case kCrossCorrNorm: return launch_typed<TYPE, CT, kCrossCorrNorm>(src, tmpl, dst, tt, st);
+    case kSqrDistance: return launch_typed<TYPE, CT, kSqrDistance>(src, tmpl, dst, tt, sms, st);
+    case kSqrDistanceNorm: return launch_typed<TYPE, CT, kSqrDistanceNorm>(src, tmpl, dst, tt, sms, st);
+    case kAbsDistance: return launch_typed<TYPE, CT, kAbsDistance>(src, tmpl, dst, tt, sms, st);
+    case kCrossCorr: return launch_typed<TYPE, CT, kCrossCorr>(src, tmpl, dst, tt, sms, st);
+    case kCrossCorrNorm: return launch_typed<TYPE, CT, kCrossCorrNorm>(src, tmpl, dst, tt, sms, st);
   }
   return cudaErrorInvalidValue;
 }
@@ -607,25 +691,25 @@ static bool small_int_exact_in_float(Measure m, int area) {
 
 cudaError_t launch_proximity_plain(Measure m, const DevImage& src,
                                    const DevImage& tmpl, const DevImage& dst,
-                                   void* tt_scratch, cudaStream_t st) {
+                                   void* tt_scratch, int sm_count, cudaStream_t st) {
   const int area = tmpl.width * tmpl.height;
   if (m == kAbsDistance && proximity_sad_8bit_supported(src, tmpl))
     return launch_proximity_sad_8bit(src, tmpl, dst, st);
   switch (src.type) {
     case U8:
       return small_int_exact_in_float(m, area)
-                 ? launch_measure<U8, float>(m, src, tmpl, dst, tt_scratch, st)
-                 : launch_measure<U8, double>(m, src, tmpl, dst, tt_scratch, st);
+                 ? launch_measure<U8, float>(m, src, tmpl, dst, tt_scratch, sm_count, st)
+                 : launch_measure<U8, double>(m, src, tmpl, dst, tt_scratch, sm_count, st);
     case S8:
       return small_int_exact_in_float(m, area)
-                 ? launch_measure<S8, float>(m, src, tmpl, dst, tt_scratch, st)
-                 : launch_measure<S8, double>(m, src, tmpl, dst, tt_scratch, st);
-    case U16: return launch_measure<U16, double>(m, src, tmpl, dst, tt_scratch, st);
-    case S16: return launch_measure<S16, double>(m, src, tmpl, dst, tt_scratch, st);
-    case U32: return launch_measure<U32, double>(m, src, tmpl, dst, tt_scratch, st);
-    case S32: return launch_measure<S32, double>(m, src, tmpl, dst, tt_scratch, st);
-    case F32: return launch_measure<F32, float>(m, src, tmpl, dst, tt_scratch, st);
-    case F64: return launch_measure<F64, double>(m, src, tmpl, dst, tt_scratch, st);
+                 ? launch_measure<S8, float>(m, src, tmpl, dst, tt_scratch, sm_count, st)
+                 : launch_measure<S8, double>(m, src, tmpl, dst, tt_scratch, sm_count, st);
+    case U16: return launch_measure<U16, double>(m, src, tmpl, dst, tt_scratch, sm_count, st);
+    case S16: return launch_measure<S16, double>(m, src, tmpl, dst, tt_scratch, sm_count, st);
+    case U32: return launch_measure<U32, double>(m, src, tmpl, dst, tt_scratch, sm_count, st);
+    case S32: return launch_measure<S32, double>(m, src, tmpl, dst, tt_scratch, sm_count, st);
+    case F32: return launch_measure<F32, float>(m, src, tmpl, dst, tt_scratch, sm_count, st);
+    case F64: return launch_measure<F64, double>(m, src, tmpl, dst, tt_scratch, sm_count, st);
   }
   return cudaErrorInvalidValue;
 }
