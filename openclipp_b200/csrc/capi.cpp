@@ -128,19 +128,16 @@ void* Context::scratch(int slot, size_t bytes) {
     }
     check_cuda(cudaMalloc(&s.ptr, bytes), "scratch allocation");
     s.bytes = bytes;
-    // New scratch starts zeroed: the kernels' error flag lives in one slot.
+    // New scratch starts zeroed: an arrival counter lives in one slot.
     check_cuda(cudaMemsetAsync(s.ptr, 0, bytes, stream), "scratch initialisation");
   }
   return s.ptr;
 }
 
 void Context::check_device_errors() {
-  const Scratch& s = scratch_[kTensorAux];
-  if (s.ptr == nullptr) return;
-  int flag = 0;
-  check_cuda(cudaMemcpy(&flag, s.ptr, sizeof(int), cudaMemcpyDeviceToHost), "error flag");
-  if (flag) {
-    check_cuda(cudaMemset(s.ptr, 0, sizeof(int)), "error flag");
+  volatile int* flag = &page->error;
+  if (*flag) {
+    *flag = 0;
     fail(CL_OUT_OF_RESOURCES,
          "a tensor-core kernel gave up a bounded wait; results since the last ocipFinish or "
          "ocipReadImage are not valid");
@@ -150,6 +147,7 @@ void Context::check_device_errors() {
 Context::~Context() {
   for (auto& s : scratch_)
     if (s.ptr) cudaFree(s.ptr);
+  if (page) cudaFreeHost(page);
   if (untracked) cudaEventDestroy(untracked);
   if (copy_stream) cudaStreamDestroy(copy_stream);
   if (stream) cudaStreamDestroy(stream);
@@ -192,10 +190,13 @@ ocipError ocipInitialize(ocipContext* ContextPtr, const char* PreferredPlatform,
     ctx->cc_minor = prop.minor;
     cudaError_t e = cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&ctx->copy_stream, cudaStreamNonBlocking);
+    if (e == cudaSuccess)
+      e = cudaHostAlloc(&ctx->page, sizeof(*ctx->page), cudaHostAllocMapped | cudaHostAllocPortable);
     if (e != cudaSuccess) {
       delete ctx;
-      check_cuda(e, "cudaStreamCreate");
+      check_cuda(e, "context creation");
     }
+    memset(ctx->page, 0, sizeof(*ctx->page));
     g_contexts[ctx] = true;
     g_current = ctx;
     *ContextPtr = reinterpret_cast<ocipContext>(ctx);

@@ -29,7 +29,7 @@ struct Context {
   enum ScratchSlot {
     kTemplateEnergy = 0,
     kPlanes = 1,
-    kTensorAux = 2,
+    kTickets = 2,        // arrival counter of the index reductions' last CTA
     kBackward = 3,
     kEnergyMap = 4,      // row energies of the tensor path
     kProductMap = 5,     // F64 product sums of templates tiled over launches
@@ -54,10 +54,24 @@ struct Context {
   int last_path = 1;  // path that served the last proximity call
   int band_rows = 0;  // output rows per tensor work item; 0: chosen per launch
   void* scratch(int slot, size_t bytes);
-  // The tensor-path kernels set a device flag (kTensorAux scratch) when a
-  // bounded wait expires (the kernel then returns without finishing its
-  // work). Called after the stream is synchronised: clears the flag and fails
-  // with CL_OUT_OF_RESOURCES if it was set.
+  // Page-locked host memory that kernels write (mapped, same address on the
+  // device): what a synchronous call needs of its kernels' results is there
+  // when the stream is synchronised, without copies of its own (each about
+  // 10 us of latency).
+  struct HostPage {
+    int error;  // a bounded wait expired
+    // Result of an index reduction.
+    struct Index {
+      float v;
+      int x, y;
+      int nan;  // a NaN score (fused best match)
+    } index;
+  };
+  HostPage* page = nullptr;
+  // The tensor-path kernels set page->error when a bounded wait expires (the
+  // kernel then returns without finishing its work). Called after the stream
+  // is synchronised: clears the flag and fails with CL_OUT_OF_RESOURCES if it
+  // was set.
   void check_device_errors();
   ~Context();
 

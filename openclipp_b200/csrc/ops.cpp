@@ -388,11 +388,10 @@ void proximity_index(int measure, int op, ocipImage hs, ocipImage ht, ocipImage 
   bool wrote_map = false;
   if (fused) {
     void* rec = ctx.scratch(Context::kIndexRecords, tensor_index_records_bytes(ctx, s, t));
-    int nrec = 0, bx = 0, by = 0;
+    int bx = 0, by = 0;
     float best = 0.f;
     bool nan = false;
-    check_cuda(launch_proximity_tensor_indexed(ctx, m, s, t, d, op, rec, &nrec, &best, &bx, &by,
-                                               &nan),
+    check_cuda(launch_proximity_tensor_indexed(ctx, m, s, t, d, op, rec, &best, &bx, &by, &nan),
                "fused best-match launch");
     ctx.last_path = OCIP_PATH_TENSOR;
     if (D) mark_written(*D);

@@ -276,7 +276,10 @@ __global__ void __launch_bounds__(kWgThreads, 1)
     tc_fence_after();
     tmem_dealloc(tmem, kWgCols);
   }
-  if (threadIdx.x == 0 && s_abort) atomicExch(p.err, 1);
+  if (threadIdx.x == 0 && s_abort) {
+    *reinterpret_cast<volatile int*>(p.err) = 1;
+    __threadfence_system();
+  }
 }
 
 // ---- Element-wise kernels ------------------------------------------------------
@@ -493,7 +496,7 @@ cudaError_t launch_wgrad(Context& ctx, const DevImage& S, int tw, int th, const 
   p.M = M;
   p.m_pitch = m_pitch;
   p.partials = partials;
-  p.err = reinterpret_cast<int*>(ctx.scratch(Context::kTensorAux, 256));
+  p.err = &ctx.page->error;
   EncodeFn enc = wg_encode();
   if (!enc) return cudaErrorNotSupported;
   CUtensorMap map;

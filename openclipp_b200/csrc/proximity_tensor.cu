@@ -1193,6 +1193,8 @@ struct TensorLaunch {
   int nbox;            // 16-byte groups per staged row (all tensor maps of the launch)
   int* err;
   // mode 0
+  unsigned* ticket;    // best match: CTAs done (0 between launches)
+  Context::HostPage::Index* index;  // and its result
   ItemArgs base;       // fields common to every item
   int BH;
   // mode 1
@@ -1205,6 +1207,72 @@ struct TensorLaunch {
   int nitems;
   int* counter;        // next item; reset to 0 before every launch
 };
+
+// Best match: the last CTA to finish folds every CTA's records (each value with
+// the smallest key among equals, so the order does not matter) into the host's
+// result.
+__device__ void fold_records(const TensorLaunch& P) {
+  __shared__ bool last;
+  __shared__ IdxRecord part[kWarps];
+  const unsigned ncta = gridDim.x * gridDim.y * gridDim.z;
+  if (threadIdx.x == 0) {
+    __threadfence();
+    last = atomicAdd(P.ticket, 1u) == ncta - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  const bool is_min = P.base.idx_op == 0 || P.base.idx_op == 2;
+  auto better = [&](float v, unsigned long long key, int have, const IdxRecord& r) {
+    return have && (!r.have || (is_min ? v < r.v : v > r.v) || (v == r.v && key < r.key));
+  };
+  IdxRecord best;
+  best.v = 0.f;
+  best.key = 0ull;
+  best.have = best.nan = best.pad = 0;
+  const IdxRecord* rec = reinterpret_cast<const IdxRecord*>(P.base.idx_out);
+  for (unsigned i = threadIdx.x; i < ncta * kEpilogue; i += kThreads) {
+    const float v = __ldcg(&rec[i].v);
+    const unsigned long long key = __ldcg(&rec[i].key);
+    const int have = __ldcg(&rec[i].have);
+    best.nan |= __ldcg(&rec[i].nan);
+    if (better(v, key, have, best)) {
+      best.v = v;
+      best.key = key;
+      best.have = 1;
+    }
+  }
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1) {
+    const float v = __shfl_xor_sync(0xffffffffu, best.v, d);
+    const unsigned long long key = __shfl_xor_sync(0xffffffffu, best.key, d);
+    const int have = __shfl_xor_sync(0xffffffffu, best.have, d);
+    best.nan |= __shfl_xor_sync(0xffffffffu, best.nan, d);
+    if (better(v, key, have, best)) {
+      best.v = v;
+      best.key = key;
+      best.have = 1;
+    }
+  }
+  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = best;
+  __syncthreads();
+  if (threadIdx.x != 0) return;
+  for (int w = 1; w < kWarps; ++w) {
+    best.nan |= part[w].nan;
+    if (better(part[w].v, part[w].key, part[w].have, best)) best = IdxRecord{part[w].v, 1, part[w].key, best.nan, 0};
+  }
+  // Key -> pixel: group, bit-reversed work-item id, pixel index in the work-item.
+  const unsigned long long grp = best.key >> 12;
+  const unsigned lid = __brev((unsigned)(best.key >> 4) & 255u) >> 24;
+  const int ngx = (P.base.W + 255) >> 8;
+  volatile Context::HostPage::Index* out = P.index;
+  out->v = best.v;
+  out->x = (int)(grp % ngx) * 256 + (int)(lid & 15) + 16 * (int)(best.key & 15);
+  out->y = (int)(grp / ngx) * 16 + (int)(lid >> 4);
+  out->nan = best.nan || !best.have;
+  __threadfence_system();
+  *P.ticket = 0;
+}
 
 // One kernel per element type. Mode 0 (one image and template): CTA
 // (x, y, z) = (strip, band, channel). Mode 1 (batch): one persistent CTA per
@@ -1292,7 +1360,11 @@ __global__ void __launch_bounds__(kThreads, 1)
     tc_fence_after();
     tmem_dealloc(cs.tmem, kTmemCols);
   }
-  if (threadIdx.x == 0 && cs.abort) atomicExch(P.err, 1);
+  if (threadIdx.x == 0 && cs.abort) {
+    *reinterpret_cast<volatile int*>(P.err) = 1;
+    __threadfence_system();
+  }
+  if (IDX) fold_records(P);
 }
 
 // Interleaved channels -> planes: plane c holds channel c of every pixel, rows
@@ -1427,7 +1499,7 @@ size_t plane_set_bytes(const DevImage& s) {
 template <int ELEM>
 cudaError_t launch_one(Context& ctx, Measure m, const DevImage& src, const DevImage& tmpl,
                        const DevImage& dst, int ax, int ay, bool accum = false,
-                       int idx_op = -1, void* idx_out = nullptr, int* nrec = nullptr) {
+                       int idx_op = -1, void* idx_out = nullptr) {
   const int cls = class_of(tmpl.height);
   const int R = class_r(cls);
   TensorLaunch P;
@@ -1435,7 +1507,7 @@ cudaError_t launch_one(Context& ctx, Measure m, const DevImage& src, const DevIm
   P.mode = 0;
   P.measure = m;
   P.nbox = nbox_for<ELEM>(cls, tmpl.width, ax);
-  P.err = reinterpret_cast<int*>(ctx.scratch(Context::kTensorAux, 256));
+  P.err = &ctx.page->error;
   const int sw = strip_width<ELEM>(cls);
   const int nstrips = (src.width + sw - 1) / sw;
   P.BH = ctx.band_rows > 0
@@ -1460,6 +1532,10 @@ cudaError_t launch_one(Context& ctx, Measure m, const DevImage& src, const DevIm
   a.accum = accum ? 1 : 0;
   a.idx_op = idx_op;
   a.idx_out = reinterpret_cast<char*>(idx_out);
+  if (idx_op >= 0) {
+    P.ticket = reinterpret_cast<unsigned*>(ctx.scratch(Context::kTickets, 256));
+    P.index = &ctx.page->index;
+  }
 
   const int smem_bytes = smem_for<ELEM>(cls, tmpl.width, ax, P.nbox);
   if (smem_bytes > kMaxDynSmem) return cudaErrorInvalidValue;
@@ -1493,7 +1569,6 @@ cudaError_t launch_one(Context& ctx, Measure m, const DevImage& src, const DevIm
                            kMaxDynSmem);
   if (e != cudaSuccess) return e;
   dim3 grid(nstrips, (src.height + P.BH - 1) / P.BH, src.nch);
-  if (nrec) *nrec = (int)(grid.x * grid.y * grid.z) * kEpilogue;
   kern<<<grid, kThreads, smem_bytes, ctx.stream>>>(P);
   count_launches(1);
   return cudaGetLastError();
@@ -1707,7 +1782,7 @@ int autotune_bh(Context& ctx, int measure, const DevImage& img, const CUtensorMa
     tb.launch.mode = 1;
     tb.launch.measure = measure;
     tb.launch.nbox = nbox;
-    tb.launch.err = reinterpret_cast<int*>(ctx.scratch(Context::kTensorAux, 256));
+    tb.launch.err = &ctx.page->error;
     tb.smem = smem;
     void* mem = nullptr;
     if (upload_tables<ELEM>(tb, maps, bimgs, btpls, bdsts, items, benergy, &mem) != cudaSuccess)
@@ -1872,7 +1947,7 @@ TensorBatch* batch_create(Context& ctx, Measure m, const std::vector<DevImage>& 
   b->launch.mode = 1;
   b->launch.measure = m;
   b->launch.nbox = b->nbox;
-  b->launch.err = reinterpret_cast<int*>(ctx.scratch(Context::kTensorAux, 256));
+  b->launch.err = &ctx.page->error;
   e = upload_tables<ELEM>(*b, maps, bimgs, btpls, bdsts, items, benergy, &b->tables);
   if (e != cudaSuccess) return fail(e);
   b->nitems = b->launch.nitems;
@@ -1909,7 +1984,10 @@ __global__ void bounded_wait_probe_kernel(long long limit, int* err) {
     mbar_init(&bar, 1);
     fence_barrier_init();
     const bool ok = mbar_wait(&bar, 0, &abort_flag, limit);
-    if (!ok) atomicExch(err, 1);
+    if (!ok) {
+      *reinterpret_cast<volatile int*>(err) = 1;
+      __threadfence_system();
+    }
     mbar_inval(&bar);
   }
 }
@@ -1917,7 +1995,7 @@ __global__ void bounded_wait_probe_kernel(long long limit, int* err) {
 }  // namespace
 
 cudaError_t launch_bounded_wait_probe(Context& ctx, long long limit_cycles) {
-  int* err = reinterpret_cast<int*>(ctx.scratch(Context::kTensorAux, 256));
+  int* err = &ctx.page->error;
   bounded_wait_probe_kernel<<<1, 32, 0, ctx.stream>>>(limit_cycles, err);
   count_launches(1);
   return cudaGetLastError();
@@ -1966,48 +2044,25 @@ size_t tensor_index_records_bytes(const Context& ctx, const DevImage& src, const
 
 cudaError_t launch_proximity_tensor_indexed(Context& ctx, Measure m, const DevImage& src,
                                             const DevImage& tmpl, const DevImage& dst, int idx_op,
-                                            void* records, int* nrec, float* best, int* bx,
-                                            int* by, bool* has_nan) {
+                                            void* records, float* best, int* bx, int* by,
+                                            bool* has_nan) {
   cudaError_t e;
   const int ax = tmpl.width / 2, ay = tmpl.height / 2;
   if (src.type == U8)
-    e = launch_one<kU8>(ctx, m, src, tmpl, dst, ax, ay, false, idx_op, records, nrec);
+    e = launch_one<kU8>(ctx, m, src, tmpl, dst, ax, ay, false, idx_op, records);
   else if (src.type == U16)
-    e = launch_one<kU16>(ctx, m, src, tmpl, dst, ax, ay, false, idx_op, records, nrec);
+    e = launch_one<kU16>(ctx, m, src, tmpl, dst, ax, ay, false, idx_op, records);
   else
-    e = launch_one<kF32>(ctx, m, src, tmpl, dst, ax, ay, false, idx_op, records, nrec);
-  if (e != cudaSuccess) return e;
-  std::vector<IdxRecord> recs(*nrec);
-  e = cudaMemcpyAsync(recs.data(), records, recs.size() * sizeof(IdxRecord),
-                      cudaMemcpyDeviceToHost, ctx.stream);
+    e = launch_one<kF32>(ctx, m, src, tmpl, dst, ax, ay, false, idx_op, records);
   if (e != cudaSuccess) return e;
   e = cudaStreamSynchronize(ctx.stream);
   if (e != cudaSuccess) return e;
-  const bool is_min = idx_op == 0 || idx_op == 2;
-  bool have = false, nan = false;
-  float v = 0.f;
-  unsigned long long key = 0;
-  for (const IdxRecord& r : recs) {
-    nan = nan || r.nan;
-    if (!r.have) continue;
-    if (!have || (is_min ? r.v < v : r.v > v) || (r.v == v && r.key < key)) {
-      v = r.v;
-      key = r.key;
-      have = true;
-    }
-  }
-  *has_nan = nan;
-  *best = v;
-  // Key -> pixel: group, bit-reversed work-item id, pixel index in the work-item.
-  const unsigned long long grp = key >> 12;
-  const unsigned rl = (unsigned)((key >> 4) & 255);  // bit-reversed work-item id
-  unsigned lid = 0;
-  for (int b = 0; b < 8; ++b) lid |= ((rl >> b) & 1u) << (7 - b);
-  const int i = (int)(key & 15);
-  const int ngx = (src.width + 255) >> 8;
-  *bx = (int)(grp % ngx) * 256 + (int)(lid & 15) + 16 * i;
-  *by = (int)(grp / ngx) * 16 + (int)(lid >> 4);
-  return have ? cudaSuccess : cudaErrorInvalidValue;
+  const volatile Context::HostPage::Index* r = &ctx.page->index;
+  *best = r->v;
+  *bx = r->x;
+  *by = r->y;
+  *has_nan = r->nan != 0;
+  return cudaSuccess;
 }
 
 cudaError_t launch_tensor_product_sums(Context& ctx, const DevImage& src, const DevImage& tmpl,

@@ -49,8 +49,8 @@ cudaError_t launch_proximity_tensor_large(Context& ctx, Measure m, const DevImag
 size_t tensor_index_records_bytes(const Context& ctx, const DevImage& src, const DevImage& tmpl);
 cudaError_t launch_proximity_tensor_indexed(Context& ctx, Measure m, const DevImage& src,
                                             const DevImage& tmpl, const DevImage& dst, int idx_op,
-                                            void* records, int* nrec, float* best, int* bx,
-                                            int* by, bool* has_nan);
+                                            void* records, float* best, int* bx, int* by,
+                                            bool* has_nan);
 
 // Gradients of L = sum G1 * SqrDistance(S, T) + sum G2 * CrossCorr_Norm(S, T)
 // (F32 sources, one channel, templates up to 64 x 64) into dS (S's size) and
