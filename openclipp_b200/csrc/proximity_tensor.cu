@@ -216,9 +216,8 @@ struct ItemArgs {
   // of R(x, r), plane ch at energy + ch * e_plane bytes, rows e_pitch apart.
   const char* energy;
   size_t e_pitch, e_plane;
-  // 1: add the scores (raw CrossCorr sums into an F64 map) to the
-  // destination instead of writing them (templates tiled over launches).
-  int accum;
+  int dst_nch, dst_ch;  // channels of the destination, and the item's
+  int raw;       // U8 product sums as int32 bits (the tiles of a larger template)
   // Best match (ocipProximityIndx): -1 none, else the index reduction
   // (0 min, 1 max, 2 min |v|, 3 max |v|) of the F32 scores; each epilogue
   // warp writes one IdxRecord per item to idx_out[item * 4 + warp]. dst may
@@ -474,30 +473,18 @@ __device__ __forceinline__ double score_d(typename Sums<SPLIT>::A cv, typename S
 // map's row: F64 maps (written or added to), several channels, the right
 // edge. v: the F32 scores, for the best match.
 template <int ELEM, int SH, int M>
-__device__ __noinline__ void store_slot(const ItemArgs& a, int ch, int xl, char* orow,
+__device__ __noinline__ void store_slot(const ItemArgs& a, int xl, char* orow,
                            const typename Sums<ElemTraits<ELEM>::split>::A* val,
                            const typename Sums<ElemTraits<ELEM>::split>::E* esum, double etd,
                            float* v) {
   constexpr bool SPLIT = ElemTraits<ELEM>::split;
   const bool u8_float = u8_norm_in_float(a.tw, a.th);
   if (a.dst_f64) {
-    double* o = reinterpret_cast<double*>(orow) + (size_t)xl * a.nch + ch;
-    if (SH > 1 && a.nch == 1 && xl + SH <= a.W) {
-#pragma unroll
-      for (int p = 0; p < SH; p += 2) {
-        double2 d = make_double2(0.0, 0.0);
-        if (a.accum) d = *reinterpret_cast<const double2*>(o + p);
-        d.x += score_d<SPLIT, M>(val[p], esum[p], etd, u8_float);
-        d.y += score_d<SPLIT, M>(val[(p + 1) % SH], esum[(p + 1) % SH], etd, u8_float);
-        *reinterpret_cast<double2*>(o + p) = d;
-      }
-      return;
-    }
+    double* o = reinterpret_cast<double*>(orow) + (size_t)xl * a.dst_nch + a.dst_ch;
 #pragma unroll
     for (int p = 0; p < SH; ++p) {
       if (xl + p >= a.W) break;
-      const double s = score_d<SPLIT, M>(val[p], esum[p], etd, u8_float);
-      o[p * a.nch] = a.accum ? o[p * a.nch] + s : s;
+      o[p * a.dst_nch] = score_d<SPLIT, M>(val[p], esum[p], etd, u8_float);
     }
     return;
   }
@@ -505,8 +492,9 @@ __device__ __noinline__ void store_slot(const ItemArgs& a, int ch, int xl, char*
 #pragma unroll
   for (int p = 0; p < SH; ++p) {
     v[p] = score_f<SPLIT, M>(val[p], esum[p], etd, ret, u8_float);
+    if (!SPLIT && a.raw) v[p] = __int_as_float(static_cast<int>(val[p]));
     if (xl + p < a.W && a.dst != nullptr)
-      reinterpret_cast<float*>(orow)[(size_t)(xl + p) * a.nch + ch] = v[p];
+      reinterpret_cast<float*>(orow)[(size_t)(xl + p) * a.dst_nch + a.dst_ch] = v[p];
   }
 }
 
@@ -535,11 +523,11 @@ __device__ __forceinline__ void run_epilogue(const ItemArgs& a, CtaState& cs, ui
   const uint32_t lane_base = tmem_base + (static_cast<uint32_t>((ew & 3) * 32) << 16);
   // The item's fields in registers: the item lives in shared memory, and
   // the score loop would otherwise reload them on every slot.
-  const int W = a.W, H = a.H, th = a.th, nch = a.nch, ch = a.ch;
+  const int W = a.W, H = a.H, th = a.th, nch = a.dst_nch;
   const int idx_op = IDX ? a.idx_op : -1;
   const int xl = a.xs_out + S * ((ew & 3) * 32 + lane) + half * SH;  // first position
   const bool whole = xl + SH <= W;
-  const bool f32 = !a.dst_f64, accum = a.accum;
+  const bool f32 = !a.dst_f64, raw = !SPLIT && a.raw;
   double etd = 0.0;  // template energy
 #pragma unroll
   for (int w = 0; w < kWarps; ++w) etd += cs.et[w];
@@ -573,7 +561,7 @@ __device__ __forceinline__ void run_epilogue(const ItemArgs& a, CtaState& cs, ui
   if (kE) {
     e_pitch = a.e_pitch;
     e_back = (size_t)th * e_pitch;
-    e_row = a.energy + (size_t)ch * a.e_plane + (size_t)xl * sizeof(RT) +
+    e_row = a.energy + (size_t)a.ch * a.e_plane + (size_t)xl * sizeof(RT) +
             (ptrdiff_t)r_begin * (ptrdiff_t)e_pitch;
   }
   auto load_row = [&](uint32_t (&v)[SH], const char* at, bool ok) {
@@ -658,19 +646,7 @@ __device__ __forceinline__ void run_epilogue(const ItemArgs& a, CtaState& cs, ui
     }
     // The block's completed slots: window energies, scores and stores.
     const bool rows = t0 >= R - 1 && t0 + BS <= nsteps;  // every slot is an output row
-    if (M == kCrossCorr && !f32 && nch == 1 && rows) {
-      // Product sums of a tile of a larger template, in an F64 map.
-#pragma unroll
-      for (int g = 0; g < BS; ++g) {
-        double* o = reinterpret_cast<double*>(orow) + xl;
-#pragma unroll
-        for (int p = 0; p < SH; ++p) {
-          const double v = (double)val[g * SH + p];
-          if (xl + p < W) o[p] = accum ? o[p] + v : v;
-        }
-        orow += dst_pitch;
-      }
-    } else if (f32 && rows) {
+    if (f32 && rows) {
       // Straight-line independent work.
       float out[8];
       ET es[8];
@@ -681,6 +657,10 @@ __device__ __forceinline__ void run_epilogue(const ItemArgs& a, CtaState& cs, ui
         es[i] = esum[p];
       }
       scores8<SPLIT, M>(out, val, es, etd, ret, u8_float);
+      if (M == kCrossCorr && raw) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) out[i] = __int_as_float(static_cast<int>(val[i]));
+      }
 #pragma unroll
       for (int g = 0; g < BS; ++g) {
         if (IDX && idx_op >= 0) {
@@ -691,7 +671,7 @@ __device__ __forceinline__ void run_epilogue(const ItemArgs& a, CtaState& cs, ui
         }
         if (IDX && !has_dst) {
         } else if (!whole || nch > 1) {
-          float* o = reinterpret_cast<float*>(orow) + (size_t)xl * nch + ch;
+          float* o = reinterpret_cast<float*>(orow) + (size_t)xl * nch + a.dst_ch;
 #pragma unroll
           for (int p = 0; p < SH; ++p)
             if (xl + p < W) o[p * nch] = out[g * SH + p];
@@ -726,7 +706,7 @@ __device__ __forceinline__ void run_epilogue(const ItemArgs& a, CtaState& cs, ui
             cv[p] = val[g * SH + p];
             ev[p] = esum[p];
           }
-          store_slot<ELEM, SH, M>(a, ch, xl, orow, cv, ev, etd, v);
+          store_slot<ELEM, SH, M>(a, xl, orow, cv, ev, etd, v);
           if (IDX && idx_op >= 0) {
 #pragma unroll
             for (int p = 0; p < SH; ++p)
@@ -1186,6 +1166,13 @@ struct BatchEnergy {
   size_t pitch, plane;
 };
 
+// A tile of a template larger than 64 x 64.
+struct TemplateTile {
+  const char* tmpl;
+  int tw, th, ax, ay;
+};
+constexpr int kMaxTiles = 16;  // of one launch
+
 struct TensorLaunch {
   CUtensorMap map;     // single-image mode: the source planes
   int mode;            // 0: one (image, template) pair, items from blockIdx; 1: work queue
@@ -1197,6 +1184,9 @@ struct TensorLaunch {
   Context::HostPage::Index* index;  // and its result
   ItemArgs base;       // fields common to every item
   int BH;
+  int ntiles;          // > 0: CTA z = (tile, channel), each with its own map of product sums
+  size_t tile_plane;   // bytes between those maps (base.dst)
+  TemplateTile tiles[kMaxTiles];
   // mode 1
   const CUtensorMap* maps;  // one per image (64-byte aligned)
   const BatchImage* imgs;
@@ -1296,7 +1286,18 @@ __global__ void __launch_bounds__(kThreads, 1)
     if (threadIdx.x == 0) {
       item = P.base;
       item.tmap = &P.map;
-      item.ch = blockIdx.z;
+      item.ch = item.dst_ch = blockIdx.z;
+      if (P.ntiles > 0) {
+        const TemplateTile t = P.tiles[blockIdx.z / item.nch];
+        item.ch = blockIdx.z % item.nch;
+        item.dst_ch = 0;
+        item.dst += blockIdx.z * P.tile_plane;
+        item.tmpl = t.tmpl;
+        item.tw = t.tw;
+        item.th = t.th;
+        item.ax = t.ax;
+        item.ay = t.ay;
+      }
       item.xs_out = blockIdx.x * kM * s_for(item.R);
       item.y0 = blockIdx.y * P.BH;
       item.yend = min(item.H, item.y0 + P.BH);
@@ -1333,7 +1334,9 @@ __global__ void __launch_bounds__(kThreads, 1)
           item.dst_pitch = ds.pitch;
           item.dst_f64 = ds.f64;
           item.measure = P.measure;
-          item.accum = 0;
+          item.dst_nch = im.nch;
+          item.dst_ch = bi.ch;
+          item.raw = 0;
           item.idx_op = -1;
           item.idx_out = nullptr;
           item.energy = nullptr;
@@ -1496,82 +1499,111 @@ size_t plane_set_bytes(const DevImage& s) {
   return pitch * s.height * s.nch;
 }
 
+// Channel planes of a source: the image itself for one channel, else a split
+// copy in the context's scratch.
+struct Planes {
+  const char* ptr;
+  size_t pitch, bytes;  // between rows, between planes
+};
+
 template <int ELEM>
-cudaError_t launch_one(Context& ctx, Measure m, const DevImage& src, const DevImage& tmpl,
-                       const DevImage& dst, int ax, int ay, bool accum = false,
-                       int idx_op = -1, void* idx_out = nullptr) {
-  const int cls = class_of(tmpl.height);
+Planes source_planes(Context& ctx, const DevImage& src) {
+  Planes p{(const char*)src.ptr, src.pitch, src.pitch * src.height};
+  if (src.nch > 1) {
+    char* pl = reinterpret_cast<char*>(ctx.scratch(Context::kPlanes, plane_set_bytes(src)));
+    p.pitch = split_channels<ELEM>(src, pl, ctx.stream);
+    p.bytes = p.pitch * src.height;
+    p.ptr = pl;
+  }
+  return p;
+}
+
+RowEnergyJob energy_job(const Planes& p, const DevImage& src, int tw, int ax, char* dst) {
+  const size_t pitch = row_energy_pitch(src.width);
+  return RowEnergyJob{p.ptr, p.pitch, p.bytes, dst, pitch, pitch * src.height, src.width,
+                      src.height, src.nch, tw, ax};
+}
+
+cudaError_t launch_energy(RowEnergyJob j, char* dst, int type, cudaStream_t stream,
+                          bool count = true) {
+  j.dst = dst;
+  if (count) count_launches(1);
+  return launch_row_energies(type, j.tw, j, nullptr, 1, j.W, j.H, stream);
+}
+
+// One launch of `n` templates of one rows class over a source: a measure's map
+// (n = 1), or the product sums of the tiles of a larger template.
+template <int ELEM>
+cudaError_t launch_items(Context& ctx, TensorLaunch& P, const DevImage& src, const Planes& planes,
+                         int cls, int n, int smem_bytes) {
+  ItemArgs& a = P.base;
   const int R = class_r(cls);
-  TensorLaunch P;
-  std::memset(&P, 0, sizeof(P));
-  P.mode = 0;
-  P.measure = m;
-  P.nbox = nbox_for<ELEM>(cls, tmpl.width, ax);
-  P.err = &ctx.page->error;
   const int sw = strip_width<ELEM>(cls);
   const int nstrips = (src.width + sw - 1) / sw;
+  P.mode = 0;
+  P.err = &ctx.page->error;
   P.BH = ctx.band_rows > 0
              ? std::min(ctx.band_rows, src.height)
-             : band_height(src.height, R, (long long)nstrips * src.nch, ctx.sm_count);
-  ItemArgs& a = P.base;
+             : band_height(src.height, R, (long long)nstrips * src.nch * n, ctx.sm_count);
   a.W = src.width;
   a.H = src.height;
-  a.tw = tmpl.width;
-  a.th = tmpl.height;
   a.R = R;
-  a.ax = ax;
-  a.ay = ay;
   a.nch = src.nch;
   a.nbox = P.nbox;
+  if (smem_bytes > kMaxDynSmem) return cudaErrorInvalidValue;
+  cudaError_t e = encode_planes<ELEM>(&P.map, planes.ptr, src.width, src.height, src.nch,
+                                      planes.pitch, planes.bytes, P.nbox);
+  if (e != cudaSuccess) return e;
+  auto kern = a.idx_op >= 0 ? prox_tensor_kernel<ELEM, true> : prox_tensor_kernel<ELEM, false>;
+  e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynSmem);
+  if (e != cudaSuccess) return e;
+  dim3 grid(nstrips, (src.height + P.BH - 1) / P.BH, src.nch * n);
+  kern<<<grid, kThreads, smem_bytes, ctx.stream>>>(P);
+  count_launches(1);
+  return cudaGetLastError();
+}
+
+template <int ELEM>
+cudaError_t launch_one(Context& ctx, Measure m, const DevImage& src, const DevImage& tmpl,
+                       const DevImage& dst, int ax, int ay, int idx_op = -1,
+                       void* idx_out = nullptr) {
+  const int cls = class_of(tmpl.height);
+  TensorLaunch P;
+  std::memset(&P, 0, sizeof(P));
+  P.measure = m;
+  P.nbox = nbox_for<ELEM>(cls, tmpl.width, ax);
+  ItemArgs& a = P.base;
+  a.tw = tmpl.width;
+  a.th = tmpl.height;
+  a.ax = ax;
+  a.ay = ay;
   a.tmpl = (const char*)tmpl.ptr;
   a.tmpl_pitch = tmpl.pitch;
   a.dst = (char*)dst.ptr;
   a.dst_pitch = dst.pitch;
   a.dst_f64 = dst.type == F64;
+  a.dst_nch = src.nch;
   a.measure = m;
-  a.accum = accum ? 1 : 0;
   a.idx_op = idx_op;
   a.idx_out = reinterpret_cast<char*>(idx_out);
   if (idx_op >= 0) {
     P.ticket = reinterpret_cast<unsigned*>(ctx.scratch(Context::kTickets, 256));
     P.index = &ctx.page->index;
   }
-
-  const int smem_bytes = smem_for<ELEM>(cls, tmpl.width, ax, P.nbox);
-  if (smem_bytes > kMaxDynSmem) return cudaErrorInvalidValue;
-
+  const Planes planes = source_planes<ELEM>(ctx, src);
   // Row energies of every source row, for the measures that use them.
   if (m != kCrossCorr) {
-    const size_t ep = row_energy_pitch(src.width);
-    const size_t eplane = ep * src.height;
-    char* emap = reinterpret_cast<char*>(ctx.scratch(Context::kEnergyMap, eplane * src.nch));
-    cudaError_t ee = launch_row_energy(src, tmpl.width, ax, emap, ep, eplane, ctx.stream);
-    if (ee != cudaSuccess) return ee;
+    const RowEnergyJob j = energy_job(planes, src, tmpl.width, ax, nullptr);
+    char* emap =
+        reinterpret_cast<char*>(ctx.scratch(Context::kEnergyMap, j.dst_plane * src.nch));
+    const cudaError_t e = launch_energy(j, emap, src.type, ctx.stream);
+    if (e != cudaSuccess) return e;
     a.energy = emap;
-    a.e_pitch = ep;
-    a.e_plane = eplane;
+    a.e_pitch = j.dst_pitch;
+    a.e_plane = j.dst_plane;
   }
-
-  // Source planes: the image itself for one channel, else a split copy.
-  const void* planes = src.ptr;
-  size_t plane_pitch = src.pitch;
-  if (src.nch > 1) {
-    char* pl = reinterpret_cast<char*>(ctx.scratch(Context::kPlanes, plane_set_bytes(src)));
-    plane_pitch = split_channels<ELEM>(src, pl, ctx.stream);
-    planes = pl;
-  }
-  cudaError_t e = encode_planes<ELEM>(&P.map, planes, src.width, src.height, src.nch,
-                                      plane_pitch, plane_pitch * src.height, P.nbox);
-  if (e != cudaSuccess) return e;
-
-  auto kern = idx_op >= 0 ? prox_tensor_kernel<ELEM, true> : prox_tensor_kernel<ELEM, false>;
-  e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           kMaxDynSmem);
-  if (e != cudaSuccess) return e;
-  dim3 grid(nstrips, (src.height + P.BH - 1) / P.BH, src.nch);
-  kern<<<grid, kThreads, smem_bytes, ctx.stream>>>(P);
-  count_launches(1);
-  return cudaGetLastError();
+  return launch_items<ELEM>(ctx, P, src, planes, cls, 1,
+                            smem_for<ELEM>(cls, tmpl.width, ax, P.nbox));
 }
 
 // ---- Batches ------------------------------------------------------------------
@@ -1599,11 +1631,10 @@ struct TensorBatch {
   std::map<int, int> bh;  // class -> band height used
   // Row-energy maps, one per (image, template width) of the batch (measures
   // other than CrossCorr), recomputed by every run.
-  struct EnergyJob {
-    int img, tw;
-    size_t offset, pitch, plane;
-  };
-  std::vector<EnergyJob> ejobs;
+  // One launch per staged width of the kernel (energy_groups) over the device
+  // table ejobs, sorted by template width.
+  std::vector<RowEnergyJob> ejobs;
+  RowEnergyJob* ejobs_dev = nullptr;
   char* emaps = nullptr;
 };
 
@@ -1618,12 +1649,22 @@ cudaError_t batch_record(TensorBatch& b, cudaStream_t stream, bool count) {
     if (b.plane_offsets[i].first)
       split_channels<ELEM>(b.images[i], b.planes + b.plane_offsets[i].second, stream, count);
   }
-  for (const TensorBatch::EnergyJob& j : b.ejobs) {
-    const unsigned long long before = g_launches;
-    cudaError_t ee = launch_row_energy(b.images[j.img], j.tw, j.tw / 2, b.emaps + j.offset,
-                                       j.pitch, j.plane, stream);
+  // Row energies: the narrow templates' maps in one launch, the others' in a
+  // second one (rows of 256 + tw - 1 pixels: 288 or 320 staged).
+  for (size_t i = 0; i < b.ejobs.size();) {
+    size_t n = i;
+    int W = 0, H = 0;
+    while (n < b.ejobs.size() && (b.ejobs[n].tw <= 33) == (b.ejobs[i].tw <= 33)) {
+      W = std::max(W, b.ejobs[n].W);
+      H = std::max(H, b.ejobs[n].H);
+      ++n;
+    }
+    const cudaError_t ee =
+        launch_row_energies(b.images[0].type, b.ejobs[n - 1].tw, b.ejobs[i], b.ejobs_dev + i,
+                            (int)(n - i), W, H, stream);
     if (ee != cudaSuccess) return ee;
-    if (!count) g_launches = before;
+    if (count) count_launches(1);
+    i = n;
   }
   cudaError_t e = cudaMemsetAsync(b.launch.counter, 0, sizeof(int), stream);
   if (e != cudaSuccess) return e;
@@ -1734,8 +1775,8 @@ cudaError_t upload_tables(TensorBatch& b, const std::vector<CUtensorMap>& maps,
 // bands) and load balance (favouring short ones).
 template <int ELEM>
 int autotune_bh(Context& ctx, int measure, const DevImage& img, const CUtensorMap& map,
-                const DevImage& tpl, int cls, int nbox, int smem, char* probe_dst,
-                size_t probe_pitch) {
+                const Planes& planes, const DevImage& tpl, int cls, int nbox, int smem,
+                char* probe_dst, size_t probe_pitch) {
   const int R = class_r(cls);
   std::vector<int> cand;
   for (int bh : {64, 128, 192, 256, 384, 512, 768, 1024})
@@ -1758,14 +1799,13 @@ int autotune_bh(Context& ctx, int measure, const DevImage& img, const CUtensorMa
   std::vector<BatchEnergy> benergy;
   char* probe_e = nullptr;
   if (measure != kCrossCorr) {
-    const size_t ep = row_energy_pitch(img.width), eplane = ep * img.height;
-    if (cudaMalloc(&probe_e, eplane * img.nch) != cudaSuccess) return cand.back();
-    if (launch_row_energy(img, tpl.width, tpl.width / 2, probe_e, ep, eplane, ctx.stream) !=
-        cudaSuccess) {
+    const RowEnergyJob j = energy_job(planes, img, tpl.width, tpl.width / 2, nullptr);
+    if (cudaMalloc(&probe_e, j.dst_plane * img.nch) != cudaSuccess) return cand.back();
+    if (launch_energy(j, probe_e, img.type, ctx.stream) != cudaSuccess) {
       cudaFree(probe_e);
       return cand.back();
     }
-    benergy.push_back(BatchEnergy{probe_e, ep, eplane});
+    benergy.push_back(BatchEnergy{probe_e, j.dst_pitch, j.dst_plane});
   }
   float best = 1e30f;
   int best_bh = cand.back();
@@ -1844,16 +1884,17 @@ TensorBatch* batch_create(Context& ctx, Measure m, const std::vector<DevImage>& 
     if (e != cudaSuccess) return fail(e);
   }
   std::vector<CUtensorMap> maps(imgs.size());
+  std::vector<Planes> planes;
   for (size_t i = 0; i < imgs.size(); ++i) {
     const DevImage& s = imgs[i];
-    const void* planes = s.ptr;
-    size_t pitch = s.pitch;
+    Planes p{(const char*)s.ptr, s.pitch, s.pitch * s.height};
     if (s.nch > 1) {
-      planes = b->planes + b->plane_offsets[i].second;
-      pitch = (plane_set_bytes(s) / s.nch) / s.height;
+      p.ptr = b->planes + b->plane_offsets[i].second;
+      p.bytes = plane_set_bytes(s) / s.nch;
+      p.pitch = p.bytes / s.height;
     }
-    e = encode_planes<ELEM>(&maps[i], planes, s.width, s.height, s.nch, pitch,
-                            pitch * s.height, b->nbox);
+    planes.push_back(p);
+    e = encode_planes<ELEM>(&maps[i], p.ptr, s.width, s.height, s.nch, p.pitch, p.bytes, b->nbox);
     if (e != cudaSuccess) return fail(e);
   }
   std::vector<BatchImage> bimgs;
@@ -1902,7 +1943,7 @@ TensorBatch* batch_create(Context& ctx, Measure m, const std::vector<DevImage>& 
     const size_t pp = ((size_t)probe.width * probe.nch * 4 + 127) / 128 * 128;
     e = cudaMalloc(&pd, pp * probe.height);
     if (e != cudaSuccess) return fail(e);
-    const int v = autotune_bh<ELEM>(ctx, m, probe, maps[0], tpls[j], cls, b->nbox,
+    const int v = autotune_bh<ELEM>(ctx, m, probe, maps[0], planes[0], tpls[j], cls, b->nbox,
                                     cls_smem[cls], pd, pp);
     cudaStreamSynchronize(ctx.stream);
     cudaFree(pd);
@@ -1919,21 +1960,31 @@ TensorBatch* batch_create(Context& ctx, Measure m, const std::vector<DevImage>& 
   std::map<std::pair<int, int>, int> eidx;
   std::vector<BatchEnergy> benergy;
   if (m != kCrossCorr) {
+    std::vector<int> widths;
+    for (const DevImage& t : tpls) widths.push_back(t.width);
+    std::sort(widths.begin(), widths.end());
+    widths.erase(std::unique(widths.begin(), widths.end()), widths.end());
     size_t total = 0;
-    for (size_t i = 0; i < imgs.size(); ++i)
-      for (const DevImage& t : tpls) {
-        const auto key = std::make_pair((int)i, t.width);
-        if (eidx.count(key)) continue;
-        eidx[key] = (int)b->ejobs.size();
-        const size_t ep = row_energy_pitch(imgs[i].width);
-        const size_t eplane = ep * imgs[i].height;
-        b->ejobs.push_back(TensorBatch::EnergyJob{(int)i, t.width, total, ep, eplane});
-        total += eplane * imgs[i].nch;
+    std::vector<size_t> at;
+    for (int w : widths)
+      for (size_t i = 0; i < imgs.size(); ++i) {
+        eidx[std::make_pair((int)i, w)] = (int)b->ejobs.size();
+        b->ejobs.push_back(energy_job(planes[i], imgs[i], w, w / 2, nullptr));
+        at.push_back(total);
+        total += b->ejobs.back().dst_plane * imgs[i].nch;
       }
     e = cudaMalloc(&b->emaps, total);
     if (e != cudaSuccess) return fail(e);
-    for (const TensorBatch::EnergyJob& j : b->ejobs)
-      benergy.push_back(BatchEnergy{b->emaps + j.offset, j.pitch, j.plane});
+    for (size_t k = 0; k < b->ejobs.size(); ++k) {
+      RowEnergyJob& j = b->ejobs[k];
+      j.dst = b->emaps + at[k];
+      benergy.push_back(BatchEnergy{j.dst, j.dst_pitch, j.dst_plane});
+    }
+    const size_t jb = b->ejobs.size() * sizeof(RowEnergyJob);
+    e = cudaMalloc(&b->ejobs_dev, jb);
+    if (e != cudaSuccess) return fail(e);
+    e = cudaMemcpy(b->ejobs_dev, b->ejobs.data(), jb, cudaMemcpyHostToDevice);
+    if (e != cudaSuccess) return fail(e);
   }
   std::vector<int> pi, pt, pd, pe;
   for (size_t i = 0; i < imgs.size(); ++i)
@@ -2049,11 +2100,11 @@ cudaError_t launch_proximity_tensor_indexed(Context& ctx, Measure m, const DevIm
   cudaError_t e;
   const int ax = tmpl.width / 2, ay = tmpl.height / 2;
   if (src.type == U8)
-    e = launch_one<kU8>(ctx, m, src, tmpl, dst, ax, ay, false, idx_op, records);
+    e = launch_one<kU8>(ctx, m, src, tmpl, dst, ax, ay, idx_op, records);
   else if (src.type == U16)
-    e = launch_one<kU16>(ctx, m, src, tmpl, dst, ax, ay, false, idx_op, records);
+    e = launch_one<kU16>(ctx, m, src, tmpl, dst, ax, ay, idx_op, records);
   else
-    e = launch_one<kF32>(ctx, m, src, tmpl, dst, ax, ay, false, idx_op, records);
+    e = launch_one<kF32>(ctx, m, src, tmpl, dst, ax, ay, idx_op, records);
   if (e != cudaSuccess) return e;
   e = cudaStreamSynchronize(ctx.stream);
   if (e != cudaSuccess) return e;
@@ -2065,13 +2116,55 @@ cudaError_t launch_proximity_tensor_indexed(Context& ctx, Measure m, const DevIm
   return cudaSuccess;
 }
 
-cudaError_t launch_tensor_product_sums(Context& ctx, const DevImage& src, const DevImage& tmpl,
-                                       const DevImage& c_map, int ax, int ay, bool accumulate) {
-  if (c_map.type != F64) return cudaErrorInvalidValue;
-  if (src.type == U8) return launch_one<kU8>(ctx, kCrossCorr, src, tmpl, c_map, ax, ay, accumulate);
-  if (src.type == U16)
-    return launch_one<kU16>(ctx, kCrossCorr, src, tmpl, c_map, ax, ay, accumulate);
-  return launch_one<kF32>(ctx, kCrossCorr, src, tmpl, c_map, ax, ay, accumulate);
+namespace {
+template <int ELEM>
+cudaError_t launch_tiles(Context& ctx, const DevImage& src, const std::vector<TensorTile>& tiles,
+                         const TensorPlanes& planes, char* maps, size_t pitch) {
+  TensorLaunch P;
+  std::memset(&P, 0, sizeof(P));
+  P.measure = kCrossCorr;
+  int rows = 0;
+  for (const TensorTile& t : tiles) rows = std::max(rows, t.tmpl.height);
+  const int cls = class_of(rows);
+  P.nbox = 1;
+  for (const TensorTile& t : tiles)
+    P.nbox = std::max(P.nbox, nbox_for<ELEM>(cls, t.tmpl.width, t.ax));
+  int smem = 0;
+  for (const TensorTile& t : tiles)
+    smem = std::max(smem, smem_for<ELEM>(cls, t.tmpl.width, t.ax, P.nbox));
+  P.ntiles = (int)tiles.size();
+  for (int i = 0; i < P.ntiles; ++i)
+    P.tiles[i] = TemplateTile{(const char*)tiles[i].tmpl.ptr, tiles[i].tmpl.width,
+                              tiles[i].tmpl.height, tiles[i].ax, tiles[i].ay};
+  P.tile_plane = pitch * src.height;
+  ItemArgs& a = P.base;
+  a.tmpl_pitch = tiles[0].tmpl.pitch;
+  a.dst = maps;
+  a.dst_pitch = pitch;
+  a.dst_nch = 1;
+  a.raw = src.type == U8;
+  a.measure = kCrossCorr;
+  a.idx_op = -1;
+  return launch_items<ELEM>(ctx, P, src, Planes{planes.ptr, planes.pitch, planes.bytes}, cls,
+                            P.ntiles, smem);
+}
+}  // namespace
+
+TensorPlanes tensor_source_planes(Context& ctx, const DevImage& src) {
+  const Planes p = src.type == U8    ? source_planes<kU8>(ctx, src)
+                   : src.type == U16 ? source_planes<kU16>(ctx, src)
+                                     : source_planes<kF32>(ctx, src);
+  return TensorPlanes{p.ptr, p.pitch, p.bytes};
+}
+
+int tensor_max_tiles() { return kMaxTiles; }
+
+cudaError_t launch_tensor_tiles(Context& ctx, const DevImage& src,
+                                const std::vector<TensorTile>& tiles, const TensorPlanes& planes,
+                                char* maps, size_t pitch) {
+  if (src.type == U8) return launch_tiles<kU8>(ctx, src, tiles, planes, maps, pitch);
+  if (src.type == U16) return launch_tiles<kU16>(ctx, src, tiles, planes, maps, pitch);
+  return launch_tiles<kF32>(ctx, src, tiles, planes, maps, pitch);
 }
 
 TensorBatch* tensor_batch_create(Context& ctx, Measure m, const std::vector<DevImage>& imgs,
@@ -2083,7 +2176,9 @@ TensorBatch* tensor_batch_create(Context& ctx, Measure m, const std::vector<DevI
 }
 
 cudaError_t tensor_batch_run(TensorBatch* b) {
-  count_launches(1 + (int)b->ejobs.size() +
+  // Launches of the graph: splits, row energies (at most two groups), the kernel.
+  const bool two = !b->ejobs.empty() && b->ejobs.front().tw <= 33 && b->ejobs.back().tw > 33;
+  count_launches(1 + (b->ejobs.empty() ? 0 : two ? 2 : 1) +
                  std::count_if(b->plane_offsets.begin(), b->plane_offsets.end(),
                                [](const std::pair<int, size_t>& p) { return p.first != 0; }));
   return cudaGraphLaunch(b->exec, b->ctx->stream);
@@ -2105,6 +2200,7 @@ void tensor_batch_destroy(TensorBatch* b) {
   if (b->tables) cudaFree(b->tables);
   if (b->planes) cudaFree(b->planes);
   if (b->emaps) cudaFree(b->emaps);
+  if (b->ejobs_dev) cudaFree(b->ejobs_dev);
   delete b;
 }
 

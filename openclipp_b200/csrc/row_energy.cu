@@ -33,16 +33,6 @@ constexpr int kWarps = 8;        // one row segment per warp
 constexpr int kSeg = 256;        // output columns per segment (8 per lane)
 constexpr int kMaxTw = 1024;  // 256 + tw - 1 <= 32 * 41
 
-struct RowEnergyParams {
-  const char* src;
-  size_t src_pitch;
-  char* dst;
-  size_t dst_pitch;   // bytes
-  size_t dst_plane;   // bytes between channel planes
-  int W, H, nch;
-  int tw, ax;
-};
-
 template <typename ET>
 struct RowSumOf {
   // Prefix sums, exact for integers: int32 for 8-bit sources (at most
@@ -53,91 +43,42 @@ struct RowSumOf {
   typedef typename std::conditional<sizeof(ET) == 1, int, float>::type R;
 };
 
-// One warp per (source row, 256 output columns). The squares of the n =
-// 256 + tw - 1 source pixels the segment's windows cover are staged in
-// shared memory (coalesced loads); lane l turns its K contiguous entries
-// into prefix sums (local prefix plus a warp scan of the lanes' totals),
-// P(i) = sum of squares [0, i) stored at entry i - 1; output column x0 + j
-// (j = lane + 32 u) is then P(j + tw) - P(j): two conflict-free reads, and
-// the warp's stores are 128-byte rows.
-template <typename ET, int K>
-__global__ void __launch_bounds__(kWarps * 32) row_energy_kernel(const RowEnergyParams p) {
-  typedef typename RowSumOf<ET>::A A;
-  typedef typename RowSumOf<ET>::R RT;
-  extern __shared__ __align__(16) unsigned char smem[];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int r = blockIdx.y * kWarps + warp;
-  if (r >= p.H) return;  // whole warp
-  const int c = blockIdx.z;
-  const int x0 = blockIdx.x * kSeg;
-  A* buf = reinterpret_cast<A*>(smem) + warp * (32 * K);
-  const ET* row = reinterpret_cast<const ET*>(p.src + (size_t)r * p.src_pitch) + c;
-  const int n = kSeg + p.tw - 1;
-  const int xs0 = x0 - p.ax;
-  // Squares of source columns xs0 .. xs0 + n - 1 (zero outside the image).
-#pragma unroll 4
-  for (int i = lane; i < 32 * K; i += 32) {
-    const int x = xs0 + i;
-    A v = A(0);
-    if (i < n && x >= 0 && x < p.W) {
-      const A e = static_cast<A>(row[x * p.nch]);
-      v = e * e;
-    }
-    buf[i] = v;
-  }
-  __syncwarp();
-  // Lane l: entries K l .. K l + K - 1 -> inclusive prefix sums in place.
-  A loc[K];
-  A tot = A(0);
-#pragma unroll
-  for (int k = 0; k < K; ++k) {
-    tot += buf[K * lane + k];
-    loc[k] = tot;
-  }
-  A incl = tot;
-#pragma unroll
-  for (int d = 1; d < 32; d <<= 1) {
-    const A o = __shfl_up_sync(0xffffffffu, incl, d);
-    if (lane >= d) incl += o;
-  }
-  const A excl = incl - tot;
-  __syncwarp();
-#pragma unroll
-  for (int k = 0; k < K; ++k) buf[K * lane + k] = excl + loc[k];
-  __syncwarp();
-  RT* dst = reinterpret_cast<RT*>(p.dst + c * p.dst_plane + (size_t)r * p.dst_pitch);
-#pragma unroll
-  for (int u = 0; u < kSeg / 32; ++u) {
-    const int j = lane + 32 * u;
-    const int x = x0 + j;
-    if (x < p.W) {
-      const A hi = buf[j + p.tw - 1];
-      const A lo = j > 0 ? buf[j - 1] : A(0);
-      dst[x] = static_cast<RT>(hi - lo);
-    }
-  }
-}
-
-// One-channel form: the segment's source pixels are staged raw with 16-byte
-// loads (from the 16-byte group at or below its first pixel, so `sh` pixels
-// lead), squared and prefix-summed in registers, and only the prefix sums
-// are written back for the differences. Same sums, in the same order, as
-// row_energy_kernel.
-template <typename ET, int K>
-__global__ void __launch_bounds__(kWarps * 32) row_energy_vec_kernel(const RowEnergyParams p) {
+// One warp per (source row, 256 output columns) of one plane of one job. The n =
+// 256 + tw - 1 source pixels the segment's windows cover are staged raw in
+// shared memory with 16-byte loads (from the 16-byte group at or below the
+// first, so `sh` pixels lead); lane l squares its K contiguous entries and
+// turns them into prefix sums (local prefix plus a warp scan of the lanes'
+// totals), P(i) = sum of squares [0, i) stored at entry i - 1; output column
+// x0 + j (j = lane + 32 u) is then P(j + tw) - P(j): two conflict-free reads,
+// and the warp's stores are 128-byte rows.
+//
+// Channels come as planes (the tensor kernels' copies): reading them
+// interleaved, one channel per block, took 96 us for 3840 x 2160 x 4 U16
+// where the planes take PLANESUS.
+// TABLE: block z takes plane z mod nch of job z / nch of a device table, else plane z
+// of the one job (a job in the kernel's parameters: 4096 x 4096 F32 took 39 us
+// with the choice made at run time, 32 without).
+template <typename ET, int K, bool TABLE>
+__global__ void __launch_bounds__(kWarps * 32)
+    row_energy_kernel(const __grid_constant__ RowEnergyJob one, const RowEnergyJob* jobs) {
   typedef typename RowSumOf<ET>::A A;
   typedef typename RowSumOf<ET>::R RT;
   constexpr int kInner = 16 / (int)sizeof(ET);                      // pixels per group
   constexpr int kRawGroups = (32 * K + kInner - 1) / kInner + 1;     // covers sh + 32 K
   extern __shared__ __align__(16) unsigned char smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  RowEnergyJob entry;
+  if (TABLE) entry = jobs[blockIdx.z / one.nch];
+  const RowEnergyJob& p = TABLE ? entry : one;
+  const int c = TABLE ? blockIdx.z % one.nch : blockIdx.z;
   const int r = blockIdx.y * kWarps + warp;
-  if (r >= p.H) return;  // whole warp
   const int x0 = blockIdx.x * kSeg;
+  if (r >= p.H || x0 >= p.W) return;  // whole warp
   A* buf = reinterpret_cast<A*>(smem) + warp * (32 * K);
   ET* raw = reinterpret_cast<ET*>(smem + (size_t)kWarps * 32 * K * sizeof(A)) +
             warp * (kRawGroups * kInner);
-  const ET* row = reinterpret_cast<const ET*>(p.src + (size_t)r * p.src_pitch);
+  const ET* row =
+      reinterpret_cast<const ET*>(p.src + c * p.src_plane + (size_t)r * p.src_pitch);
   const int n = kSeg + p.tw - 1;
   const int xs0 = x0 - p.ax;
   const int xa = xs0 >= 0 ? xs0 - xs0 % kInner : -((-xs0 + kInner - 1) / kInner) * kInner;
@@ -178,7 +119,7 @@ __global__ void __launch_bounds__(kWarps * 32) row_energy_vec_kernel(const RowEn
 #pragma unroll
   for (int k = 0; k < K; ++k) buf[K * lane + k] = excl + loc[k];
   __syncwarp();
-  RT* dst = reinterpret_cast<RT*>(p.dst + (size_t)r * p.dst_pitch);
+  RT* dst = reinterpret_cast<RT*>(p.dst + c * p.dst_plane + (size_t)r * p.dst_pitch);
 #pragma unroll
   for (int u = 0; u < kSeg / 32; ++u) {
     const int j = lane + 32 * u;
@@ -191,69 +132,64 @@ __global__ void __launch_bounds__(kWarps * 32) row_energy_vec_kernel(const RowEn
   }
 }
 
+// `n` jobs (a device table), or the one given.
 template <typename ET, int K>
-cudaError_t launch_k(const RowEnergyParams& p, cudaStream_t st) {
+cudaError_t launch_k(const RowEnergyJob& one, const RowEnergyJob* jobs, int n, int W, int H,
+                     cudaStream_t st) {
   typedef typename RowSumOf<ET>::A A;
-  if (p.nch == 1 && (p.src_pitch % 16) == 0 && ((uintptr_t)p.src % 16) == 0) {
-    constexpr int kInner = 16 / (int)sizeof(ET);
-    constexpr int kRawGroups = (32 * K + kInner - 1) / kInner + 1;
-    const size_t smem = (size_t)kWarps * (32 * K * sizeof(A) + kRawGroups * 16);
-    auto kern = row_energy_vec_kernel<ET, K>;
+  constexpr int kInner = 16 / (int)sizeof(ET);
+  constexpr int kRawGroups = (32 * K + kInner - 1) / kInner + 1;
+  const size_t smem = (size_t)kWarps * (32 * K * sizeof(A) + kRawGroups * 16);
+  auto launch = [&](auto kern, dim3 grid, const RowEnergyJob* table) {
     if (smem > 48 * 1024) {
       const cudaError_t e =
           cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
       if (e != cudaSuccess) return e;
     }
-    dim3 grid((p.W + kSeg - 1) / kSeg, (p.H + kWarps - 1) / kWarps, 1);
-    kern<<<grid, kWarps * 32, smem, st>>>(p);
-    count_launches(1);
+    kern<<<grid, kWarps * 32, smem, st>>>(one, table);
     return cudaGetLastError();
-  }
-  const size_t smem = (size_t)kWarps * 32 * K * sizeof(A);
-  auto kern = row_energy_kernel<ET, K>;
-  if (smem > 48 * 1024) {
-    const cudaError_t e =
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  };
+  const unsigned nx = (W + kSeg - 1) / kSeg, ny = (H + kWarps - 1) / kWarps;
+  if (!jobs) return launch(row_energy_kernel<ET, K, false>, dim3(nx, ny, one.nch), nullptr);
+  // Grid dimension z holds 65535 planes.
+  const int most = 65535 / one.nch;
+  for (int i = 0; i < n; i += most) {
+    const cudaError_t e = launch(row_energy_kernel<ET, K, true>,
+                                 dim3(nx, ny, one.nch * (n - i < most ? n - i : most)), jobs + i);
     if (e != cudaSuccess) return e;
   }
-  dim3 grid((p.W + kSeg - 1) / kSeg, (p.H + kWarps - 1) / kWarps, p.nch);
-  kern<<<grid, kWarps * 32, smem, st>>>(p);
-  count_launches(1);
-  return cudaGetLastError();
+  return cudaSuccess;
+}
+
+// Staged entries per lane for a template width: 32 K >= 256 + tw - 1.
+constexpr int k_for(int tw) {
+  const int n = kSeg + tw - 1;
+  return n <= 32 * 9 ? 9 : n <= 32 * 11 ? 11 : n <= 32 * 17 ? 17 : 41;
 }
 
 template <typename ET>
-cudaError_t launch_typed(const RowEnergyParams& p, cudaStream_t st) {
-  // K: staged entries per lane, 32 K >= 256 + tw - 1.
-  const int n = kSeg + p.tw - 1;
-  if (n <= 32 * 9) return launch_k<ET, 9>(p, st);
-  if (n <= 32 * 11) return launch_k<ET, 11>(p, st);
-  if (n <= 32 * 17) return launch_k<ET, 17>(p, st);
-  return launch_k<ET, 41>(p, st);
+cudaError_t launch_typed(int tw, const RowEnergyJob& one, const RowEnergyJob* jobs, int n, int W,
+                         int H, cudaStream_t st) {
+  switch (k_for(tw)) {
+    case 9: return launch_k<ET, 9>(one, jobs, n, W, H, st);
+    case 11: return launch_k<ET, 11>(one, jobs, n, W, H, st);
+    case 17: return launch_k<ET, 17>(one, jobs, n, W, H, st);
+    default: return launch_k<ET, 41>(one, jobs, n, W, H, st);
+  }
 }
 
 }  // namespace
 
 size_t row_energy_pitch(int width) { return ((size_t)width * 4 + 127) / 128 * 128; }
 
-cudaError_t launch_row_energy(const DevImage& src, int tw, int ax, void* dst, size_t dst_pitch,
-                              size_t dst_plane, cudaStream_t stream) {
-  if (tw < 1 || tw > kMaxTw) return cudaErrorInvalidValue;
-  RowEnergyParams p;
-  p.src = (const char*)src.ptr;
-  p.src_pitch = src.pitch;
-  p.dst = (char*)dst;
-  p.dst_pitch = dst_pitch;
-  p.dst_plane = dst_plane;
-  p.W = src.width;
-  p.H = src.height;
-  p.nch = src.nch;
-  p.tw = tw;
-  p.ax = ax;
-  switch (src.type) {
-    case U8: return launch_typed<uint8_t>(p, stream);
-    case U16: return launch_typed<uint16_t>(p, stream);
-    case F32: return launch_typed<float>(p, stream);
+cudaError_t launch_row_energies(int type, int tw_max, const RowEnergyJob& one,
+                                const RowEnergyJob* jobs, int n, int W, int H,
+                                cudaStream_t stream) {
+  if (tw_max < 1 || tw_max > kMaxTw) return cudaErrorInvalidValue;
+  switch (type) {
+    case U8: return launch_typed<uint8_t>(tw_max, one, jobs, n, W, H, stream);
+    case U16: return launch_typed<uint16_t>(tw_max, one, jobs, n, W, H, stream);
+    case F32: return launch_typed<float>(tw_max, one, jobs, n, W, H, stream);
     default: return cudaErrorInvalidValue;
   }
 }

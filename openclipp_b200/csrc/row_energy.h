@@ -1,20 +1,31 @@
-// Row-energy maps for the tensor-core ImageProximity path.
+// Row energies of the ImageProximity windows (row_energy.cu).
 #pragma once
 
 #include <cuda_runtime.h>
-
-#include "internal.h"
+#include <stddef.h>
 
 namespace ocipb {
 
-// Row pitch (bytes) of a row-energy plane of the given width (4-byte entries).
+// Row pitch (bytes) of a row-energy map: 4 bytes per column, 128-byte rows.
 size_t row_energy_pitch(int width);
 
-// R(x, r, c) = sum_{w < tw} S(x + w - ax, r, c)^2 (zero outside the image) for
-// every output column x and source row r, written to dst + c * dst_plane +
-// r * dst_pitch (bytes): int32 for U8 sources (exact), FP32 for U16 and F32
-// sources (FP64 sums rounded once). tw <= 1024.
-cudaError_t launch_row_energy(const DevImage& src, int tw, int ax, void* dst, size_t dst_pitch,
-                              size_t dst_plane, cudaStream_t stream);
+// R(x, r) = sum_{w < tw} S(x + w - ax, r)^2 (zero outside the image) of every
+// plane of an image: int32 for U8, FP32 for U16 and F32. Source rows start on
+// 16 bytes.
+struct RowEnergyJob {
+  const char* src;
+  size_t src_pitch, src_plane;  // bytes between rows, between channel planes
+  char* dst;
+  size_t dst_pitch, dst_plane;
+  int W, H, nch;
+  int tw, ax;
+};
+
+// One launch for the job `one` (jobs null, n = 1) or for `n` jobs of a device
+// table with one type and channel count (one.nch): W, H and tw_max are the
+// largest of any job.
+cudaError_t launch_row_energies(int type, int tw_max, const RowEnergyJob& one,
+                                const RowEnergyJob* jobs, int n, int W, int H,
+                                cudaStream_t stream);
 
 }  // namespace ocipb

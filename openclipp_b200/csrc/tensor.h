@@ -24,18 +24,30 @@ cudaError_t launch_proximity_tensor_anchored(Context& ctx, Measure m, const DevI
                                              const DevImage& tmpl, const DevImage& dst, int ax,
                                              int ay);
 
-// Product sums C(x, y) = sum_{w, h} S(x + w - ax, y + h - ay) T(w, h) of one
-// template of at most 64 x 64 (a tile of a larger one) on the tensor cores,
-// written into (accumulate = false) or added to (true) the F64 map c_map of
-// the source's size and channels. Any anchor, including ones outside the
-// template (a tile's offset within the whole template).
-cudaError_t launch_tensor_product_sums(Context& ctx, const DevImage& src, const DevImage& tmpl,
-                                       const DevImage& c_map, int ax, int ay, bool accumulate);
+// Product sums C(x, y) = sum_{w, h} S(x + w - ax, y + h - ay) T(w, h) of up to
+// tensor_max_tiles() templates of at most 64 x 64 (tiles of a larger one, with any
+// anchor, including ones outside the template: a tile's offset within the whole
+// template) in one launch: tile i and channel c into the map at
+// maps + (i nch + c) * pitch * height, FP32 (split sources) or int32 (U8).
+struct TensorTile {
+  DevImage tmpl;
+  int ax, ay;
+};
+// Channel planes of a source (the image itself, or a split copy in scratch).
+struct TensorPlanes {
+  const char* ptr;
+  size_t pitch, bytes;  // between rows, between planes
+};
+TensorPlanes tensor_source_planes(Context& ctx, const DevImage& src);
+int tensor_max_tiles();
+cudaError_t launch_tensor_tiles(Context& ctx, const DevImage& src,
+                                const std::vector<TensorTile>& tiles, const TensorPlanes& planes,
+                                char* maps, size_t pitch);
 
 // A measure of a template larger than 64 x 64 (up to 1024 columns): the
-// template is cut into tiles of at most 64 x 64 whose product sums accumulate
-// in an F64 map, and a scoring pass adds the window energies (row energies
-// plus running column sums) and the template energy.
+// template is cut into tiles of at most 64 x 64, each with a map of its product
+// sums, and a scoring pass adds those up in FP64, with the window energies (row
+// energies plus running column sums) and the template energy.
 cudaError_t launch_proximity_tensor_large(Context& ctx, Measure m, const DevImage& src,
                                           const DevImage& tmpl, const DevImage& dst);
 
