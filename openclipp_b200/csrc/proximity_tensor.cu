@@ -582,6 +582,9 @@ __device__ __forceinline__ void run_epilogue(const ItemArgs& a, CtaState& cs, ui
   for (int c = 0; c < kRingChunks; ++c)
 #pragma unroll
     for (int j = 0; j < 8; ++j) ring[c][j] = AT(0);
+  // The row energies come from the launch before this one, which this kernel
+  // may overlap up to here (launch_items).
+  if (kE) cudaGridDependencySynchronize();
   char* orow = a.dst + (ptrdiff_t)(a.y0 - R + 1) * (ptrdiff_t)a.dst_pitch;  // of slot 0
   const size_t dst_pitch = a.dst_pitch;
   const bool has_dst = a.dst != nullptr;
@@ -1532,7 +1535,14 @@ cudaError_t launch_energy(RowEnergyJob j, char* dst, int type, cudaStream_t stre
 }
 
 // One launch of `n` templates of one rows class over a source: a measure's map
-// (n = 1), or the product sums of the tiles of a larger template.
+// (n = 1), or the product sums of the tiles of a larger template. With row
+// energies the kernel is a programmatic dependent of the launch that writes
+// them (the one before it on the stream): it starts as that one's blocks leave,
+// and only the epilogue waits for the energies, so its start (TMEM, template
+// operand, first rows: 6 us) runs in the tail of that launch. Whatever was on
+// the stream before the energies has completed, as that launch is an ordinary
+// one. 1920 x 1080 U8 48 x 40 CrossCorr_Norm 73.9 -> 70.6 us, 4096 x 4096 F32 31 x 31
+// 214 -> 211.
 template <int ELEM>
 cudaError_t launch_items(Context& ctx, TensorLaunch& P, const DevImage& src, const Planes& planes,
                          int cls, int n, int smem_bytes) {
@@ -1557,10 +1567,19 @@ cudaError_t launch_items(Context& ctx, TensorLaunch& P, const DevImage& src, con
   auto kern = a.idx_op >= 0 ? prox_tensor_kernel<ELEM, true> : prox_tensor_kernel<ELEM, false>;
   e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynSmem);
   if (e != cudaSuccess) return e;
-  dim3 grid(nstrips, (src.height + P.BH - 1) / P.BH, src.nch * n);
-  kern<<<grid, kThreads, smem_bytes, ctx.stream>>>(P);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(nstrips, (src.height + P.BH - 1) / P.BH, src.nch * n);
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = smem_bytes;
+  cfg.stream = ctx.stream;
+  cudaLaunchAttribute attr = {};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = a.energy ? 1 : 0;
+  e = cudaLaunchKernelEx(&cfg, kern, P);
   count_launches(1);
-  return cudaGetLastError();
+  return e != cudaSuccess ? e : cudaGetLastError();
 }
 
 template <int ELEM>

@@ -69,6 +69,7 @@ __global__ void __launch_bounds__(kWarps * 32)
   constexpr int kRawGroups = (32 * K + kInner - 1) / kInner + 1;     // covers sh + 32 K
   extern __shared__ __align__(16) unsigned char smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  cudaTriggerProgrammaticLaunchCompletion();  // the tensor kernel may start in the tail
   RowEnergyJob entry;
   if (TABLE) entry = jobs[blockIdx.z / one.nch];
   const RowEnergyJob& p = TABLE ? entry : one;
