@@ -40,14 +40,22 @@
 // accumulate, which clears the buffer. Partial buffers are double-buffered: the
 // epilogue reads block k while the tensor cores fill block k + 1.
 //
-// Running sums. The epilogue adds each block's partials to the running sums of
-// the open slots, 64 registers of each thread (FP32 round-to-nearest, exact
-// int32 for U8). The first 8 columns of a half are the B slots the block
+// Running sums, F32 and U16. The epilogue adds each block's partials to the running sums of
+// the open slots, 64 registers of each thread (FP32 round-to-nearest). The first 8 columns of a half are the B slots the block
 // completes; the sums move down 8 registers a block as they are added to. The
 // tensor cores' FP32 accumulation into one value thus never spans more than
 // one block: that accumulator rounds every addition with a bias that grows with
 // the number of additions, so the chains of a whole window (th rows x K
 // chunks) would cost accuracy.
+//
+// U8. Integer sums are exact in any order, so they need neither partials nor running
+// sums: the MMAs accumulate in TMEM over the whole window, in a ring of 512 columns
+// that a block's 144-column window moves along by 16 columns (in two parts where it
+// wraps; the slots then stand S columns each, without halves). The epilogue takes
+// the 16 columns that a block completes and clears them; the MMAs may run up to 24
+// blocks ahead of it, and the row energies of blocks of 2 or 4 steps are fetched
+// three blocks ahead. A batch of 60 U8 maps of 1024 x 1024 (templates of 8 to 64 a
+// side, SqrDistance) went from 426 to 381 us.
 //
 // Window energies sum S^2 of each position (measures other than CrossCorr):
 // a separate pre-pass (row_energy.cu) writes the row energies R(x, r) =
@@ -119,6 +127,14 @@ constexpr int kHalf = kHalfN + 8;       // columns of a half: a block's slides f
 constexpr int kNp = 2 * kHalf;          // MMA N
 constexpr int kPartCols = kNp;          // TMEM columns per partial buffer (two of them)
 constexpr int kRingChunks = kHalfN / 8; // open slots of a half: 8 chunks of 8 columns
+// U8: the sums of all open slots accumulate in TMEM, in a ring of 32 chunks of 16
+// columns; a block's MMAs cover 9 of them.
+constexpr int kU8Chunks = 32, kU8Window = kNp / 16, kU8Group = 8, kU8Groups = kU8Chunks / kU8Group;
+constexpr int kMaxBlk = kU8Chunks;      // "block full" barriers at most
+// U8: row energies of the next blocks on their way in shared memory (2 KB a warp and
+// block). The MMAs of a block of 2 to 8 steps take less than a load's latency.
+constexpr int kU8Ahead = 4;
+constexpr int kU8Energies = 2048;
 constexpr int kTmemCols = 512;
 constexpr int kMinSmem = 120 * 1024;    // keeps one CTA per SM (it takes all of TMEM)
 constexpr int kMaxDynSmem = 226 * 1024; // opt-in dynamic shared memory limit of the kernel
@@ -170,7 +186,7 @@ __host__ __device__ inline Geo make_geo(bool split, int R, int tw, int lead) {
   g.Q = 16 / g.S;
   g.R = R;
   g.B = block_steps(g.S);
-  g.NB = kNp + 8 - g.S / 2;
+  g.NB = split ? kNp + 8 - g.S / 2 : kNp + 16 - g.S;
   const int cmk = split ? 8 : 16;
   const int keff = tw + g.S - 1 + lead;
   g.KC = (keff + cmk - 1) / cmk;
@@ -245,7 +261,7 @@ struct IdxRecord {
 
 // Shared-memory layout, identical on host and device.
 struct Layout {
-  int row_bytes, raw_stage, raw, b, a_stage, a, bars, total;
+  int row_bytes, raw_stage, raw, b, a_stage, a, energies, bars, total;
 };
 
 __host__ __device__ inline int align128(int x) { return (x + 127) & ~127; }
@@ -267,9 +283,10 @@ __host__ __device__ inline Layout make_layout(bool split, const Geo& g, int nbox
   L.b = L.raw + raw_stages(split) * L.raw_stage;
   L.a = L.b + align128(2 * g.nmma * g.NB * 16);
   L.a_stage = align128(g.QR * 16 * (split ? 2 : 1));
-  L.bars = L.a + g.NA * L.a_stage;
-  // raw full; A block ready, A block free; block full, buffer free; done.
-  L.total = L.bars + align128(8 * (kMaxRaw + 2 * kMaxAB + 4 + 1));
+  L.energies = L.a + g.NA * L.a_stage;
+  L.bars = L.energies + (split ? 0 : kEpilogue * kU8Ahead * kU8Energies);
+  // raw full; A block ready, A block free; block full, sums read; done.
+  L.total = L.bars + align128(8 * (kMaxRaw + 2 * kMaxAB + kMaxBlk + kU8Groups + 1));
   return L;
 }
 
@@ -508,12 +525,15 @@ __device__ __noinline__ void store_slot(const ItemArgs& a, int xl, char* orow,
 template <int ELEM, int S, bool IDX, int M>
 __device__ __forceinline__ void run_epilogue(const ItemArgs& a, CtaState& cs, uint32_t tmem_base,
                                              uint64_t* blk_full, uint64_t* buf_free, int r_begin,
-                                             int nsteps) {
+                                             int nsteps, unsigned char* energies) {
   constexpr bool SPLIT = ElemTraits<ELEM>::split;
   constexpr int R = kSR / S;
   constexpr int BS = block_steps(S);
   constexpr int SH = S / 2;
   constexpr bool kE = M != kCrossCorr;  // the measure needs window energies
+  // U8 blocks of 2 and 4 steps: energies fetched blocks ahead. Blocks of 8 steps last
+  // long enough (1920 x 1080 48 x 40 took 72.1 us with it, 70.6 without).
+  constexpr bool kAhead = kE && !SPLIT && S > 2;
   typedef typename Sums<SPLIT>::A AT;
   typedef typename Sums<SPLIT>::E ET;
   typedef typename Sums<SPLIT>::R RT;
@@ -575,22 +595,51 @@ __device__ __forceinline__ void run_epilogue(const ItemArgs& a, CtaState& cs, ui
       v[0] = ok ? *reinterpret_cast<const uint32_t*>(at) : 0u;
     }
   };
-  // Running sums of the open slots (FP32 round-to-nearest, exact int32 for U8):
-  // 8 chunks of BS slots, chunk 0 the next block's completed one.
-  AT ring[kRingChunks][8];
+  // Running sums of the open slots (FP32 round-to-nearest): 8 chunks of BS slots,
+  // chunk 0 the next block's completed one.
+  // U8: they are in TMEM.
+  AT ring[SPLIT ? kRingChunks : 1][8];
+  if constexpr (SPLIT) {
 #pragma unroll
-  for (int c = 0; c < kRingChunks; ++c)
+    for (int c = 0; c < kRingChunks; ++c)
 #pragma unroll
-    for (int j = 0; j < 8; ++j) ring[c][j] = AT(0);
+      for (int j = 0; j < 8; ++j) ring[c][j] = AT(0);
+  }
   // The row energies come from the launch before this one, which this kernel
   // may overlap up to here (launch_items).
   if (kE) cudaGridDependencySynchronize();
   char* orow = a.dst + (ptrdiff_t)(a.y0 - R + 1) * (ptrdiff_t)a.dst_pitch;  // of slot 0
   const size_t dst_pitch = a.dst_pitch;
   const bool has_dst = a.dst != nullptr;
+  // U8: block k's row energies by cp.async into slot k mod kU8Ahead, each lane its
+  // own (entering rows, then leaving ones), one commit group a block.
+  auto slot_of = [&](int k, int i) {
+    return reinterpret_cast<uint32_t*>(energies + (ew * kU8Ahead + k % kU8Ahead) * kU8Energies) +
+           (i * 32 + lane) * SH;
+  };
+  auto prefetch = [&](int k) {
+    if (k * BS < nsteps) {
+#pragma unroll
+      for (int g = 0; g < BS; ++g) {
+        const int u = k * BS + g, r = r_begin + u;
+        const bool in = u < nsteps && xl < W;
+        const char* at = e_row + g * e_pitch;
+        const bool enter = in && r >= 0 && r < H, leave = in && u >= th && r >= th && r - th < H;
+        cp_async_zfill<4 * SH>(slot_of(k, g), enter ? at : a.energy, enter);
+        cp_async_zfill<4 * SH>(slot_of(k, BS + g), leave ? at - e_back : a.energy, leave);
+      }
+      e_row += BS * e_pitch;
+    }
+    cp_async_commit();
+  };
+  if constexpr (kAhead) {
+#pragma unroll
+    for (int k = 0; k < kU8Ahead - 1; ++k) prefetch(k);
+  }
   for (int k = 0; k * BS < nsteps; ++k) {
     const int t0 = k * BS;
-    if (kE) {
+    if constexpr (kAhead) prefetch(k + kU8Ahead - 1);
+    if (kE && !kAhead) {
 #pragma unroll
       for (int g = 0; g < BS; ++g) {
         const int u = t0 + g, r = r_begin + u;
@@ -600,45 +649,72 @@ __device__ __forceinline__ void run_epilogue(const ItemArgs& a, CtaState& cs, ui
       }
       e_row += BS * e_pitch;
     }
-    const bool ok = mbar_wait(&blk_full[k & 1], (k >> 1) & 1, abort_flag, kSpinLimit);
+    constexpr int NBLK = SPLIT ? 2 : kU8Chunks;
+    const bool ok = mbar_wait(&blk_full[k % NBLK], (k / NBLK) & 1, abort_flag, kSpinLimit);
     // tcgen05.ld/st are warp-collective: the whole warp takes one branch.
     if (!__all_sync(0xffffffffu, ok)) break;
     tc_fence_after();
-    const uint32_t part = lane_base + (k & 1) * kPartCols + half * kHalf;
-    // Chunk 0 of the partial completes the BS slots t0 .. t0 + BS - 1; chunk c
-    // belongs to the open sums c - 1 of the next block (the sums move down a
-    // chunk as they are added to). Three chunks are in flight together.
     AT val[8];
-    auto chunks = [&](auto first) {
-      constexpr int C0 = decltype(first)::value, N = 3;
-      uint32_t vp[N][8];
+    if constexpr (SPLIT) {
+      const uint32_t part = lane_base + (k & 1) * kPartCols + half * kHalf;
+      // Chunk 0 of the partial completes the BS slots t0 .. t0 + BS - 1; chunk c
+      // belongs to the open sums c - 1 of the next block (the sums move down a
+      // chunk as they are added to). Three chunks are in flight together.
+      auto chunks = [&](auto first) {
+        constexpr int C0 = decltype(first)::value, N = 3;
+        uint32_t vp[N][8];
 #pragma unroll
-      for (int c = 0; c < N; ++c) tmem_ld8x(part + 8 * (C0 + c), vp[c]);
+        for (int c = 0; c < N; ++c) tmem_ld8x(part + 8 * (C0 + c), vp[c]);
+        tmem_ld_wait();
+#pragma unroll
+        for (int c = 0; c < N; ++c)
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            const AT old = C0 + c < kRingChunks ? ring[(C0 + c) % kRingChunks][j] : AT(0);
+            const AT v = __fadd_rn(old, __uint_as_float(vp[c][j]));
+            if (C0 + c == 0)
+              val[j] = v;
+            else
+              ring[(C0 + c + kRingChunks - 1) % kRingChunks][j] = v;
+          }
+      };
+      chunks(std::integral_constant<int, 0>());
+      chunks(std::integral_constant<int, 3>());
+      chunks(std::integral_constant<int, 6>());
+      // The partial has been read: the MMAs may refill it (block k + 2).
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&buf_free[k & 1]);
+    } else {
+      // The chunk of the block's BS completed slots, column S g + p; this warp
+      // takes its half of the positions and clears those columns for the slots
+      // 512 / S later.
+      const uint32_t chunk = lane_base + 16 * (k % kU8Chunks);
+      uint32_t v[16];
+      tmem_ld16x(chunk, v);
       tmem_ld_wait();
 #pragma unroll
-      for (int c = 0; c < N; ++c)
+      for (int g = 0; g < BS; ++g) {
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const AT old = C0 + c < kRingChunks ? ring[(C0 + c) % kRingChunks][j] : AT(0);
-          AT v;
-          if constexpr (SPLIT)
-            v = __fadd_rn(old, __uint_as_float(vp[c][j]));
-          else
-            v = old + static_cast<int>(vp[c][j]);  // exact int32 sums
-          if (C0 + c == 0)
-            val[j] = v;
-          else
-            ring[(C0 + c + kRingChunks - 1) % kRingChunks][j] = v;
-        }
-    };
-    chunks(std::integral_constant<int, 0>());
-    chunks(std::integral_constant<int, 3>());
-    chunks(std::integral_constant<int, 6>());
-    // The partial has been read: the MMAs may refill it (block k + 2).
-    tc_fence_before();
-    __syncwarp();
-    if (lane == 0) mbar_arrive(&buf_free[k & 1]);
-    if (kE) {
+        for (int p = 0; p < SH; ++p)
+          val[g * SH + p] = static_cast<int>(half ? v[S * g + SH + p] : v[S * g + p]);
+        tmem_st_zero<SH>(chunk + S * g + SH * half);
+      }
+      tmem_st_wait();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&buf_free[(k / kU8Group) % kU8Groups]);
+    }
+    if constexpr (kAhead) {
+      cp_async_wait<kU8Ahead - 1>();
+#pragma unroll
+      for (int g = 0; g < BS; ++g) {
+        memcpy(rin[g], __builtin_assume_aligned(slot_of(k, g), 4 * SH), 4 * SH);
+        memcpy(rout[g], __builtin_assume_aligned(slot_of(k, BS + g), 4 * SH), 4 * SH);
+      }
+      __syncwarp();
+    }
+    if (kE && !kAhead) {
       // The loaded energies are first used here: without this the compiler
       // converts them where they were loaded, and waits for the loads there
       // (about 900 cycles a step).
@@ -721,6 +797,7 @@ __device__ __forceinline__ void run_epilogue(const ItemArgs& a, CtaState& cs, ui
       }
     }
   }
+  if (kAhead) cp_async_wait<0>();  // none is left in flight after a wait that gave up
   if (IDX && idx_op >= 0) {
     // The warp's best: same rule, then lane 0 writes the warp's record.
     const bool is_min = idx_op == 0 || idx_op == 2;
@@ -776,9 +853,11 @@ __device__ __forceinline__ void run_item(const ItemArgs& a, unsigned char* smem,
   // the builders may refill them (block k + AB).
   uint64_t* ready = raw_full + kMaxRaw;
   uint64_t* a_free = ready + kMaxAB;
-  uint64_t* blk_full = a_free + kMaxAB;    // block's MMAs complete (2 buffers)
-  uint64_t* buf_free = blk_full + 2;       // block's buffer read by the epilogue
-  uint64_t* done_bar = buf_free + 2;
+  uint64_t* blk_full = a_free + kMaxAB;    // block's MMAs complete (a buffer or chunk each)
+  uint64_t* buf_free = blk_full + kMaxBlk;  // block's buffer read by the epilogue; U8: the
+                                            // chunks of a group of 8 blocks read and cleared
+  uint64_t* done_bar = buf_free + kU8Groups;
+  constexpr int NBLK = SPLIT ? 2 : kU8Chunks, NFREE = SPLIT ? 2 : kU8Groups;
   volatile int* abort_flag = &cs.abort;
 
   const int warp = threadIdx.x >> 5;
@@ -794,10 +873,8 @@ __device__ __forceinline__ void run_item(const ItemArgs& a, unsigned char* smem,
       mbar_init(&ready[i], BS);
       mbar_init(&a_free[i], 1);
     }
-    for (int i = 0; i < 2; ++i) {
-      mbar_init(&blk_full[i], 1);
-      mbar_init(&buf_free[i], kEpilogue);
-    }
+    for (int i = 0; i < NBLK; ++i) mbar_init(&blk_full[i], 1);
+    for (int i = 0; i < NFREE; ++i) mbar_init(&buf_free[i], SPLIT ? kEpilogue : kEpilogue * kU8Group);
     mbar_init(done_bar, 1);
     fence_barrier_init();
   }
@@ -861,12 +938,15 @@ __device__ __forceinline__ void run_item(const ItemArgs& a, unsigned char* smem,
     // Template operand B: per core matrix (two per MMA, in issue order) NB rows
     // of 16 bytes, a thread per row; rows zp .. zp + 63 hold the first half of the positions,
     // rows zp + 72 .. zp + 135 the second, the rest are zero.
-    constexpr int zp = 8 - SH;
+    // U8: rows zp + S j + p, slot after slot.
+    constexpr int zp = SPLIT ? 8 - SH : 16 - S;
     constexpr int NB = kNp + zp;
     const int total = 2 * G.nmma * NB;
     for (int idx = threadIdx.x; idx < total; idx += kThreads) {
       const int cm = idx / NB, r = idx - cm * NB - zp;
-      const int half = r >= kHalf, n = r - half * kHalf;  // row of its half
+      const int half = SPLIT && r >= kHalf;
+      const int n = r - half * kHalf;        // row of its half (U8: of all)
+      constexpr int rows = SPLIT ? SH : S;   // rows of a slot
       // Which part (0 zero, 1 Thi, 2 Tlo; U8: 1) and which K chunk.
       int part, c;
       if (SPLIT) {
@@ -882,11 +962,11 @@ __device__ __forceinline__ void run_item(const ItemArgs& a, unsigned char* smem,
         c = cm;
         part = c < G.KC ? 1 : 0;
       }
-      const int h = a.th - 1 - n / SH;
+      const int h = a.th - 1 - n / rows;
       uint4 q = make_uint4(0u, 0u, 0u, 0u);
-      if (part && n >= 0 && n < kHalfN && h >= 0) {
+      if (part && n >= 0 && n < (SPLIT ? kHalfN : kN) && h >= 0) {
         // Elements w = c CMK - p - lead .. + CMK - 1 of template row h.
-        const int at = h * tpitch + c * CMK + S - 1 - (half * SH + n % SH);
+        const int at = h * tpitch + c * CMK + S - 1 - (half * SH + n % rows);
         uint32_t w4[4];
         if (SPLIT) {
           const uint16_t* st =
@@ -904,9 +984,25 @@ __device__ __forceinline__ void run_item(const ItemArgs& a, unsigned char* smem,
       }
       *reinterpret_cast<uint4*>(smem + L.b + idx * 16) = q;
     }
+    if constexpr (!SPLIT) {
+      // Every MMA accumulates: the ring of sums starts at zero (each epilogue warp
+      // clears half of the columns of its lanes).
+      if (warp >= kFirstEpilogue) {
+        const int ew = warp - kFirstEpilogue;
+        const uint32_t at = cs.tmem + (static_cast<uint32_t>((ew & 3) * 32) << 16) + (ew >> 2) * 256;
+        uint32_t zero[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) zero[i] = 0u;
+#pragma unroll 4
+        for (int i = 0; i < 256; i += 16) tmem_st16(at + i, zero);
+        tmem_st_wait();
+      }
+    }
     // B is complete, and the staged template read, for the MMA and builder warps.
     fence_async_smem();
+    tc_fence_before();
     __syncthreads();
+    tc_fence_after();
   }
   const uint32_t tmem_base = cs.tmem;
 
@@ -919,7 +1015,7 @@ __device__ __forceinline__ void run_item(const ItemArgs& a, unsigned char* smem,
     // a wait per step and descriptors in per-lane registers an MMA went out
     // every 95-130 cycles; this form measured 73-76 (steps of 8 MMAs).
     {
-      const uint32_t idesc = SPLIT ? idesc_bf16_f32(kM, kNp) : idesc_u8_s32(kM, kNp);
+      const uint32_t idesc = idesc_bf16_f32(kM, kNp);
       auto uniform = [](uint32_t v) { return __shfl_sync(0xffffffffu, v, 0); };
       const uint32_t tm = uniform(tmem_base);
       const uint32_t a0 = uniform(smem_u32(smem + L.a));
@@ -932,12 +1028,23 @@ __device__ __forceinline__ void run_item(const ItemArgs& a, unsigned char* smem,
                 nb = uniform(nblk);
       const bool issuer = elect_one();
       for (int k = 0; k < nb; ++k) {
-        // The buffer of block k was read by the epilogue (block k - 2).
-        bool ok = k < 2 || mbar_wait(&buf_free[k & 1], ((k >> 1) - 1) & 1, abort_flag, kSpinLimit);
+        // The buffer of block k was read by the epilogue (block k - 2). U8: the chunks
+        // that the next 8 blocks' windows reach for the first time were cleared (the
+        // blocks 24 to 17 back).
+        bool ok = true;
+        if (SPLIT) {
+          ok = k < 2 || mbar_wait(&buf_free[k & 1], ((k >> 1) - 1) & 1, abort_flag, kSpinLimit);
+        } else if (k % kU8Group == 0 && k >= 3 * kU8Group) {
+          const int g = k / kU8Group - 3;
+          ok = mbar_wait(&buf_free[g % kU8Groups], (g / kU8Groups) & 1, abort_flag, kSpinLimit);
+        }
         ok = ok && mbar_wait(&ready[k % AB], (k / AB) & 1, abort_flag, kSpinLimit);
         if (!__all_sync(0xffffffffu, ok)) break;
         tc_fence_after();
         const uint32_t d = tm + (k & 1) * kPartCols;  // the block's partial
+        // U8: its window of the ring, in two parts where it wraps.
+        const int c0 = k % kU8Chunks, n1 = min(kU8Window, kU8Chunks - c0);
+        const uint32_t id1 = idesc_u8_s32(kM, 16 * n1), id2 = idesc_u8_s32(kM, kNp - 16 * n1);
         if (issuer) {
 #pragma unroll
           for (int q = 0; q < BS; ++q) {
@@ -946,7 +1053,7 @@ __device__ __forceinline__ void run_item(const ItemArgs& a, unsigned char* smem,
               // Descriptors advance by one add of their low word per MMA: B by
               // two core matrices, A by one (split, hi/lo pairs) or two K core
               // matrices. The block's first MMA overwrites all kNp columns.
-              uint32_t bl = desc_lo(b0 + 16 * SH * (BS - 1 - q), bstride);
+              uint32_t bl = desc_lo(b0 + 16 * (SPLIT ? SH : S) * (BS - 1 - q), bstride);
               uint32_t acc = q == 0 ? 0u : 1u;
               if (SPLIT) {
                 uint32_t al = desc_lo(ah, a_hl);
@@ -963,10 +1070,11 @@ __device__ __forceinline__ void run_item(const ItemArgs& a, unsigned char* smem,
                   bl += bstep;
                 }
               } else {
+                (void)acc;
                 uint32_t al = desc_lo(ah, lbok);
                 for (int j = 0; j < nmma; ++j) {
-                  mma_i8_h(d, al, dhi, bl, dhi, idesc, acc);
-                  acc = 1u;
+                  mma_i8_h(tm + 16 * c0, al, dhi, bl, dhi, id1, 1u);
+                  if (n1 < kU8Window) mma_i8_h(tm, al, dhi, bl + 16 * n1, dhi, id2, 1u);
                   al += 2 * astep;
                   bl += bstep;
                 }
@@ -974,7 +1082,7 @@ __device__ __forceinline__ void run_item(const ItemArgs& a, unsigned char* smem,
             }
           }
           // The block's partial for the epilogue, its A stages for the builders.
-          mma_commit(&blk_full[k & 1]);
+          mma_commit(&blk_full[k % NBLK]);
           // (The last blocks' stages are not refilled: no arrival is left pending.)
           if (k + AB < nb) mma_commit(&a_free[k % AB]);
         }
@@ -1093,17 +1201,20 @@ __device__ __forceinline__ void run_item(const ItemArgs& a, unsigned char* smem,
     const uint32_t tm = tmem_base;
     switch (a.measure) {
       case kSqrDistance:
-        run_epilogue<ELEM, S, IDX, kSqrDistance>(a, cs, tm, blk_full, buf_free, r_begin, nsteps);
+        run_epilogue<ELEM, S, IDX, kSqrDistance>(a, cs, tm, blk_full, buf_free, r_begin, nsteps,
+                                                smem + L.energies);
         break;
       case kSqrDistanceNorm:
         run_epilogue<ELEM, S, IDX, kSqrDistanceNorm>(a, cs, tm, blk_full, buf_free, r_begin,
-                                                     nsteps);
+                                                     nsteps, smem + L.energies);
         break;
       case kCrossCorrNorm:
-        run_epilogue<ELEM, S, IDX, kCrossCorrNorm>(a, cs, tm, blk_full, buf_free, r_begin, nsteps);
+        run_epilogue<ELEM, S, IDX, kCrossCorrNorm>(a, cs, tm, blk_full, buf_free, r_begin, nsteps,
+                                                   smem + L.energies);
         break;
       default:
-        run_epilogue<ELEM, S, IDX, kCrossCorr>(a, cs, tm, blk_full, buf_free, r_begin, nsteps);
+        run_epilogue<ELEM, S, IDX, kCrossCorr>(a, cs, tm, blk_full, buf_free, r_begin, nsteps,
+                                                smem + L.energies);
         break;
     }
   }
@@ -1117,10 +1228,8 @@ __device__ __forceinline__ void run_item(const ItemArgs& a, unsigned char* smem,
       mbar_inval(&ready[i]);
       mbar_inval(&a_free[i]);
     }
-    for (int i = 0; i < 2; ++i) {
-      mbar_inval(&blk_full[i]);
-      mbar_inval(&buf_free[i]);
-    }
+    for (int i = 0; i < NBLK; ++i) mbar_inval(&blk_full[i]);
+    for (int i = 0; i < NFREE; ++i) mbar_inval(&buf_free[i]);
     mbar_inval(done_bar);
   }
 }

@@ -100,6 +100,24 @@ __device__ __forceinline__ void fence_async_smem() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
 
+// ---- cp.async ---------------------------------------------------------------
+
+// BYTES (4, 8 or 16) from global to shared memory; zeros when `ok` is false
+// (nothing is read then, whatever `src` is).
+template <int BYTES>
+__device__ __forceinline__ void cp_async_zfill(void* dst, const void* src, bool ok) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"(smem_u32(dst)), "l"(src),
+               "n"(BYTES), "r"(ok ? BYTES : 0)
+               : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() {
+  asm volatile("cp.async.commit_group;" ::: "memory");
+}
+template <int N>
+__device__ __forceinline__ void cp_async_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
 // ---- TMA --------------------------------------------------------------------
 
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int x, int y,
@@ -288,6 +306,21 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t* v) {
       "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]),
       "r"(v[15])
       : "memory");
+}
+
+// Zeroes N (1, 2 or 4) consecutive 32-bit TMEM columns of this thread's lane.
+template <int N>
+__device__ __forceinline__ void tmem_st_zero(uint32_t taddr) {
+  if constexpr (N == 1)
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x1.b32 [%0], {%1};" ::"r"(taddr), "r"(0u)
+                 : "memory");
+  else if constexpr (N == 2)
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x2.b32 [%0], {%1,%1};" ::"r"(taddr), "r"(0u)
+                 : "memory");
+  else
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1,%1,%1,%1};" ::"r"(taddr),
+                 "r"(0u)
+                 : "memory");
 }
 
 // Stores 4 / 8 consecutive 32-bit TMEM columns of this thread's lane.

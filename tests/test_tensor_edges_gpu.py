@@ -42,6 +42,19 @@ def test_u8_edges_equal_plain(ocip, ctx, th, dw, band):
             assert np.array_equal(plain, got, equal_nan=True), (m, dtype)
 
 
+@pytest.mark.parametrize("th", [12, 32, 64])
+@pytest.mark.parametrize("H", [190, 255, 700])
+def test_u8_tall_bands_equal_plain(ocip, ctx, th, H):
+    """One band: its blocks go round the ring of sums in tensor memory (32 blocks of 2, 4 or 8 rows)
+    up to ten times."""
+    rng = np.random.default_rng(th + H)
+    S = rng.integers(0, 256, (H, 300), dtype=np.uint8)
+    T = rng.integers(0, 256, (th, 31), dtype=np.uint8)
+    for m in MEAS:
+        plain, got = both(ocip, ctx, m, S, T, np.float32, H)
+        assert np.array_equal(plain, got, equal_nan=True), m
+
+
 @pytest.mark.parametrize("th,tw", [(17, 17), (40, 48), (64, 64)])
 def test_u8_norm_rounding_equals_plain(ocip, ctx, th, tw):
     rng = np.random.default_rng(th)
