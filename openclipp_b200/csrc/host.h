@@ -5,6 +5,7 @@
 
 #include <cstdint>
 #include <map>
+#include <mutex>
 #include <new>
 #include <string>
 
@@ -81,6 +82,11 @@ struct Context {
     size_t bytes = 0;
   };
   Scratch scratch_[kNumScratch];
+
+ public:
+  // Held from an index reduction's launch until its result has been read from
+  // the page: calls of several threads (each with its own program) share it.
+  std::mutex index_mutex;
 };
 
 // Counterpart of the reference's Image (C++/Image.cpp:154-166) over a Buffer

@@ -338,6 +338,7 @@ void index_op(int op, ocipProgram hp, ocipImage hs, double* result, int* x, int*
     prog.scratch_bytes = need;
   }
   send_if_needed(S);
+  std::lock_guard<std::mutex> lock(ctx.index_mutex);
   check_cuda(index_reduce(ctx, op, dev_view(S), prog.scratch, result, x, y), "index reduction");
   ctx.check_device_errors();
 }
@@ -386,6 +387,7 @@ void proximity_index(int measure, int op, ocipImage hs, ocipImage ht, ocipImage 
   const bool fused = ctx.path != OCIP_PATH_PLAIN && t.width <= 64 && t.height <= 64 &&
                      tensor_supports(m, s, t, d, ctx.path == OCIP_PATH_TENSOR);
   bool wrote_map = false;
+  std::lock_guard<std::mutex> lock(ctx.index_mutex);
   if (fused) {
     void* rec = ctx.scratch(Context::kIndexRecords, tensor_index_records_bytes(ctx, s, t));
     int bx = 0, by = 0;
