@@ -189,6 +189,11 @@ cudaError_t launch_row_energies(int type, int tw_max, const RowEnergyJob& one,
                                 const RowEnergyJob* jobs, int n, int W, int H,
                                 cudaStream_t stream) {
   if (tw_max < 1 || tw_max > kMaxTw) return cudaErrorInvalidValue;
+  // The kernels read 16-byte groups of pixels and write 4-byte sums. (A table's
+  // planes have passed the check that its tensor maps make.)
+  if (!jobs && (((uintptr_t)one.src | one.src_pitch | one.src_plane) % 16 ||
+                ((uintptr_t)one.dst | one.dst_pitch | one.dst_plane) % 4))
+    return cudaErrorInvalidValue;
   switch (type) {
     case U8: return launch_typed<uint8_t>(tw_max, one, jobs, n, W, H, stream);
     case U16: return launch_typed<uint16_t>(tw_max, one, jobs, n, W, H, stream);
