@@ -40,6 +40,7 @@ namespace {
 
 constexpr int WCH = 8;    // template columns per inner step
 constexpr int kSmemBudget = 200 * 1024;
+constexpr int kHalfSm = 113 * 1024;  // shared memory of a CTA that leaves room for another
 
 template <int TYPE> struct ElemOf;
 template <> struct ElemOf<U8> { typedef uint8_t T; };
@@ -212,11 +213,20 @@ __device__ __forceinline__ void apply_chunk(CT (&acc)[RX], CT (&acc2)[RX],
   }
 }
 
+// FP64, 8 x 1 outputs a thread: the kernels that would take 130 to 137 registers, so
+// that no second CTA shares the SM, are held to 128 (no spills; 2306 x 2107 S16 18 x 4
+// CrossCorr_Norm 152 -> 103 us). The others take 112 to 128 by themselves; held to it they were
+// up to 5 percent slower (512 x 512 U16 31 x 31 CrossCorr 43.1 -> 44.9 us).
+__host__ __device__ constexpr bool over_half(int type, int meas) {
+  return meas == kSqrDistanceNorm || (meas == kCrossCorrNorm && (type == U16 || type == S16));
+}
+
 // NW warps of RY output rows each. TYPE: the source type, or -1 for p.type.
 // KT: for the packed FP32 form, the columns of the template's last chunk,
 // tw - WCH * ((tw - 1) / WCH), in 1 .. WCH; 0 for the other forms.
 template <int TYPE, typename CT, int MEAS, int RX, int RY, int NW, int KT>
-__global__ void __launch_bounds__(NW * 32, sizeof(CT) == 4 ? 16 / NW : 1)
+__global__ void __launch_bounds__(NW * 32, sizeof(CT) == 4 ? 16 / NW
+                                           : RY == 1 && over_half(TYPE, MEAS) ? 2 : 1)
     prox_plain_kernel(const PlainParams p) {
   constexpr int kThreads = NW * 32;
   constexpr int TX = 32 * RX;
@@ -545,6 +555,15 @@ __global__ void __launch_bounds__(256) template_energy_kernel(const char* tmpl, 
   if (threadIdx.x == 0) out[c] = s;
 }
 
+// Shared memory of a CTA whose tile has TY rows, with rb source rows staged at a time.
+template <typename CT, int RX, int TY, bool PACKED>
+size_t tile_bytes(int tw, int th, int rb) {
+  const int twp = (tw + WCH - 1) / WCH * WCH;
+  const int tb = std::min(th, rb + TY - 1);
+  return (size_t)rb * row_bytes_for<CT, RX>(32 * RX + twp) +
+         (size_t)tb * twp * sizeof(CT) * (PACKED ? 2 : 1);
+}
+
 // NW warps of RY rows a CTA: the launch of one measure.
 template <int TYPE, typename CT, int MEAS, int RX, int RY, int NW>
 cudaError_t launch_tiled(const DevImage& src, const DevImage& tmpl, const DevImage& dst,
@@ -577,10 +596,7 @@ cudaError_t launch_tiled(const DevImage& src, const DevImage& tmpl, const DevIma
   const int qtot = TY + p.th - 1;
   // Band size: all rows if they fit, else as many as the budget allows.
   int RB = qtot;
-  auto bytes_for = [&](int rb) {
-    const int tb = std::min(p.th, rb + TY - 1);
-    return (size_t)rb * p.rowBytes + (size_t)tb * p.twp * sizeof(CT) * (kPacked ? 2 : 1);
-  };
+  auto bytes_for = [&](int rb) { return tile_bytes<CT, RX, TY, kPacked>(p.tw, p.th, rb); };
   while (RB > 1 && bytes_for(RB) > (size_t)kSmemBudget) RB = (RB + 1) / 2;
   if (bytes_for(RB) > (size_t)kSmemBudget) return cudaErrorInvalidValue;
   p.RB = RB;
@@ -642,10 +658,18 @@ cudaError_t launch_tiled(const DevImage& src, const DevImage& tmpl, const DevIma
 // F32 31 x 31 AbsDistance 82.3, 89.0, 84.1; 2048 x 2048 F32 31 x 31 CrossCorr 187,
 // 209, 218.
 //
-// FP64: 256 x 8 (8 warps of 8 x 1): half the accumulators of 8 x 2, so that two
-// CTAs share an SM. 512 x 512 U16 31 x 31 CrossCorr 68.0 -> 43.4 us, 1500 x 1300
-// U8 31 x 31 CrossCorr 262 -> 222, 1920 x 1080 U16 31 x 31 SqrDistance 349 -> 335
-// (640 x 480 U8 31 x 31 SqrDistance_Norm 127 -> 139: 180 tiles, two rounds).
+// FP64: 256 x 16 (8 warps of 8 x 2) uses each window register for two rows, and one CTA
+// takes an SM; 256 x 8 (8 x 1) fits twice, one CTA's arithmetic over the other's staging,
+// where its shared memory is at most half of the SM's (templates of up to 31 to 40 rows). A
+// window load (32 wavefronts of a warp) then feeds half the arithmetic, and alone on an SM
+// the form is bound by those loads. Time per output against 256 x 16 on a full chip: 0.7
+// (few taps) to 1.0 for two CTAs, 0.9 here; 1.1 to 1.3 for one, 1.16 here. Two CTAs that are
+// an SM's only ones have nothing to stage behind the arithmetic: 0.9 of one tall tile with
+// 280 to 340 taps, 1.0 with 450, 1.04 with 600 to 1500. The tile with the least time on the
+// busiest SM is taken. Measured, us, 256 x 16 and 256 x 8: 512 x
+// 512 U16 31 x 31 CrossCorr 65.7, 43.1; 2048 x 2048 U8 64 x 64 CrossCorr 1795, 2192; 1920 x
+// 1080 U8 48 x 40 CrossCorr_Norm 673, 775; 1280 x 720 U16 9 x 40 CrossCorr 84, 105; 1024 x
+// 1024 U16 16 x 16 SqrDistance_Norm 74, 70; 4096 x 4096 U16 9 x 9 AbsDistance 436, 316.
 template <int TYPE, typename CT, int MEAS>
 cudaError_t launch_typed(const DevImage& src, const DevImage& tmpl,
                          const DevImage& dst, void* tt_buf, int sm_count, cudaStream_t st) {
@@ -663,6 +687,18 @@ cudaError_t launch_typed(const DevImage& src, const DevImage& tmpl,
     if (mid < large) return launch_tiled<TYPE, CT, MEAS, 4, 2, 8>(src, tmpl, dst, tt_buf, st);
     return launch_tiled<TYPE, CT, MEAS, 8, 4, 8>(src, tmpl, dst, tt_buf, st);
   } else {
+    auto rows = [&](int ty) {
+      const long long tiles =
+          (long long)((src.width + 255) / 256) * ((src.height + ty - 1) / ty) * src.nch;
+      return (double)((tiles + sm_count - 1) / sm_count) * ty;
+    };
+    const int tw = tmpl.width, th = tmpl.height;
+    const bool two = tile_bytes<CT, 8, 8, false>(tw, th, th + 7) <= (size_t)kHalfSm;
+    const double low = !two ? 1.16 : rows(16) == 16 && tw * th > 450 ? 1.02 : 0.9;
+    // (Rows too wide for the tall tile's share of the template take the other.)
+    if (rows(16) <= rows(8) * low &&
+        tile_bytes<CT, 8, 16, false>(tw, th, 1) <= (size_t)kSmemBudget)
+      return launch_tiled<TYPE, CT, MEAS, 8, 2, 8>(src, tmpl, dst, tt_buf, st);
     return launch_tiled<TYPE, CT, MEAS, 8, 1, 8>(src, tmpl, dst, tt_buf, st);
   }
 }
