@@ -29,7 +29,6 @@ inline int type_bytes(int t) {
   return (t >= 0 && t < 8) ? b[t] : 0;
 }
 inline bool type_is_float(int t) { return t == F32 || t == F64; }
-inline bool type_is_unsigned(int t) { return t == U8 || t == U16 || t == U32; }
 
 // Device view of an image: `nch` interleaved channels of `type` per pixel,
 // rows `pitch` bytes apart.

@@ -67,7 +67,6 @@ struct PlainParams {
   int tw, th, twp;
   int rowBytes;     // bytes per shared-memory source row (with pad chunks)
   int RB;           // source rows per band
-  int TB;           // template rows per band
   int nbands;
 };
 
@@ -600,7 +599,6 @@ cudaError_t launch_tiled(const DevImage& src, const DevImage& tmpl, const DevIma
   while (RB > 1 && bytes_for(RB) > (size_t)kSmemBudget) RB = (RB + 1) / 2;
   if (bytes_for(RB) > (size_t)kSmemBudget) return cudaErrorInvalidValue;
   p.RB = RB;
-  p.TB = std::min(p.th, RB + TY - 1);
   p.nbands = (qtot + RB - 1) / RB;
   const size_t smem = bytes_for(RB);
 

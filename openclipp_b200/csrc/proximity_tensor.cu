@@ -168,7 +168,7 @@ __host__ __device__ constexpr int block_steps(int S) { return 16 / S; }
 
 // Geometry of one work item (host and device).
 struct Geo {
-  int S, P, Q, R, B;
+  int S, P, R, B;
   int NB;          // B-operand rows stored per core matrix
   int KC;          // core matrices of one K segment
   int nmma;        // MMAs per source row
@@ -183,7 +183,6 @@ __host__ __device__ inline Geo make_geo(bool split, int R, int tw, int lead) {
   Geo g;
   g.S = s_for(R);
   g.P = kM * g.S;
-  g.Q = 16 / g.S;
   g.R = R;
   g.B = block_steps(g.S);
   g.NB = split ? kNp + 8 - g.S / 2 : kNp + 16 - g.S;
@@ -314,8 +313,6 @@ __device__ __forceinline__ float tmpl_at(const ItemArgs& a, int h, int w, int c)
   if (ELEM == kU16) return __ldg(reinterpret_cast<const uint16_t*>(row) + i);
   return __ldg(reinterpret_cast<const uint8_t*>(row) + i);
 }
-
-__host__ __device__ constexpr int ilog2(int x) { return x <= 1 ? 0 : 1 + ilog2(x / 2); }
 
 // S staged elements from element e0, a multiple of S, as floats (F32, U16).
 template <int ELEM, int S>
