@@ -33,7 +33,7 @@ struct Context {
     kTickets = 2,        // arrival counter of the index reductions' last CTA
     kBackward = 3,
     kEnergyMap = 4,      // row energies of the tensor path
-    kProductMap = 5,     // F64 product sums of templates tiled over launches
+    kProductMap = 5,     // product sums of large templates' tiles, 4 bytes (and FP64 sums of groups)
     kTemplateStats = 6,  // per-channel template energy (FP64)
     kIndexRecords = 7,   // per-warp best-match records of the fused reduction
     kIndexMap = 8,       // score map of ocipProximityIndx when no Dest is given

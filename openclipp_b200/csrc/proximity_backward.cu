@@ -645,8 +645,8 @@ cudaError_t proximity_backward(Context& ctx, const DevImage& S, const DevImage& 
                                const DevImage* dS, const DevImage* dT) {
   const int W = S.width, H = S.height, tw = T.width, th = T.height;
   const int ax = tw / 2, ay = th / 2;
-  // Scratch: row window sums HS2 / HP and the map P (FP64), M and Q (F32),
-  // flipped template, template energy and sums, weight-gradient partials.
+  // Scratch: the map P (FP64), M and Q (F32), flipped template, template energy,
+  // weight-gradient partials, the blocks' sums.
   const size_t p8 = pitch_of(W, 8), p4 = pitch_of(W, 4);
   const size_t tfp = pitch_of(tw, 4);
   const int PR = tw <= 32 ? 4 : 2;

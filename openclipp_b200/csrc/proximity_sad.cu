@@ -11,8 +11,9 @@
 // absolute differences of two packed words (bytes unsigned for U8, signed for
 // S8) to a 32-bit sum.
 //
-// Tiling follows the plain kernel: a CTA of 8 warps owns a 256 x 32 output
-// tile; lane l owns 8 consecutive columns, warp w owns 4 consecutive rows.
+// Tiling follows the plain kernel: a CTA of 8 warps owns a 256 x 32 output tile, one
+// of 2 warps (small images) a 256 x 8 one; lane l owns 8 consecutive columns, warp w
+// owns 4 consecutive rows.
 // The tile's source rows (plus halo) and the template rows are staged in
 // shared memory as bytes (one channel of the interleaved pixels, zero outside
 // the image; template rows zero-padded to a multiple of 8). For each source

@@ -60,13 +60,14 @@
 // Window energies sum S^2 of each position (measures other than CrossCorr):
 // a separate pre-pass (row_energy.cu) writes the row energies R(x, r) =
 // sum_{w < tw} S^2(x + w - ax, r) of every source row (int32 for U8, FP32
-// otherwise); the epilogue keeps each position's window energy as an FP64
-// running sum over the rows it walks (add R of the row a slot completes,
-// drop R of the row th back), loading a block's R values before it waits for
-// the block's MMAs. Exact for U8; 2^-24 relative for F32 and U16.
-// SqrDistance = E_S - 2C + E_T and the _Norm scale are done in FP64 (F32,
-// U16) or as the plain path does them (U8: the results are bit-identical to
-// it).
+// otherwise); the epilogue keeps each position's window energy as a running
+// sum (FP64; int32 for U8) over the rows it walks (add R of the row a slot
+// completes, drop R of the row th back), loading a block's R values before it
+// waits for the block's MMAs. Exact for U8; for F32 and U16 one rounding of
+// 2^-24 per row energy, as far as row_energy.cu states. F32 and U16 sources:
+// SqrDistance = E_S - 2C + E_T is formed in FP64, the _Norm scale in FP32 for
+// an F32 map and in FP64 for an F64 one. U8: as the plain path does them (the
+// results are bit-identical to it).
 //
 // Roles (12 warps; one CTA per SM, which holds all 512 TMEM columns):
 //   warps 0-2  builders: each loads (TMA, zero fill outside the image) and
@@ -234,8 +235,8 @@ struct ItemArgs {
   int dst_nch, dst_ch;  // channels of the destination, and the item's
   int raw;       // U8 product sums as int32 bits (the tiles of a larger template)
   // Best match (ocipProximityIndx): -1 none, else the index reduction
-  // (0 min, 1 max, 2 min |v|, 3 max |v|) of the F32 scores; each epilogue
-  // warp writes one IdxRecord per item to idx_out[item * 4 + warp]. dst may
+  // (0 min, 1 max, 2 min |v|, 3 max |v|) of the F32 scores; each epilogue warp
+  // writes one IdxRecord per item to idx_out[item * kEpilogue + warp]. dst may
   // then be null (no map written).
   int idx_op;
   char* idx_out;
@@ -484,8 +485,7 @@ __device__ __forceinline__ double score_d(typename Sums<SPLIT>::A cv, typename S
 }
 
 // Scores and stores of one slot that is not a whole run of a one-channel F32
-// map's row: F64 maps (written or added to), several channels, the right
-// edge. v: the F32 scores, for the best match.
+// map's row: F64 maps, several channels, the right edge. v: the F32 scores, for the best match.
 template <int ELEM, int SH, int M>
 __device__ __noinline__ void store_slot(const ItemArgs& a, int xl, char* orow,
                            const typename Sums<ElemTraits<ELEM>::split>::A* val,
@@ -514,7 +514,8 @@ __device__ __noinline__ void store_slot(const ItemArgs& a, int xl, char* orow,
 
 // Epilogue of an item, one of two warps of each TMEM sub-partition: warp
 // 4 + 4 h + s takes positions [h S/2, (h + 1) S/2) of lanes 32 s .. 32 s + 31,
-// which have their own 72 columns of the partials and of the ring. One warp is
+// which have their own 72 columns of the partials (U8: S/2 of every S columns of the
+// ring). One warp is
 // a chain of dependent steps (TMEM round trips, conversions, energies), so
 // the block's time is its latency; with one warp per sub-partition, FP64
 // scores of every measure and a wait per 16 columns, the 31 x 31 F32 kernel's

@@ -7,15 +7,19 @@
 // (cl-files/ImageProximityFFT.cl:55-84) and of the sum S^2 accumulator of
 // the direct _Norm kernels (cl-files/ImageProximity.cl:122-211, 375-466) --
 // is then the sum of R over the th rows y - ay .. y - ay + th - 1, which the
-// tensor kernel's epilogue keeps as a running FP64 sum while it walks down
-// the rows. Rows are independent here, so every warp streams its own row
+// tensor kernel's epilogue keeps as a running sum (FP64; int32 for U8) while it
+// walks down the rows. Rows are independent here, so every warp streams its own row
 // segment with all its loads in flight.
 //
 // R is stored as FP32 for F32 and U16 sources (a difference of FP64 prefix
-// sums rounded once: relative error 2^-24; an FP64 running sum of FP32
-// values adds and later removes each value exactly) and as int32 for U8
-// sources (exact). Bound: HBM (the source read once, 4 bytes written per
-// output column and source row).
+// sums rounded once: 2^-24 of it and, for F32, about 2^-50 of its segment's
+// energy) and as int32 for U8 sources (exact). An FP64 running sum of FP32
+// values adds and later removes each value exactly while their exponents lie
+// within 2^29 of one another, less log2 th: always for U16, and for F32 down to
+// energies of about 2^-24 of the brightest window's. Beyond that an F32 window can
+// keep a residue of what is beside or above it, up to 2^-50 of that energy (a
+// window of zeros a finite score instead of NaN). Bound: HBM (the source read
+// once, 4 bytes written per output column and source row).
 #include <cuda_runtime.h>
 
 #include <algorithm>

@@ -9,8 +9,8 @@
 // take more than kMapBytes), each writing a map of its own: FP32 sums, or int32
 // (i8 MMA, exact). The scoring pass adds the tiles' sums in FP64, in tile order,
 // and forms the measure from them, the window energy (the row energies of
-// row_energy.cu summed over th rows as a running FP64 sum down each column)
-// and the template energy, with the same formulas as the one-launch kernel's
+// row_energy.cu summed in FP64 over th rows, by blocks of 16 output rows) and
+// the template energy, with the same formulas as the one-launch kernel's
 // epilogue: U8 results are bit-identical to the plain path's, F32 and U16
 // within its split-BF16 error.
 //
