@@ -80,12 +80,15 @@
 // Bound: an MMA of M = 128, N = 144 takes the tensor pipe 72 cycles and reads
 // 8.7 KB of operands from shared memory in them, 120 of the 128 bytes a cycle
 // that shared memory and L1 give, so what the other warps read and write there
-// (staged rows, A operand, energies, maps) slows the MMAs: the 31 x 31 F32
-// step of 8 MMAs (576 cycles) takes 870 (CrossCorr) to 1060 (with energies);
-// it took 1150 to 1290 with a wait per step, one warp per sub-partition in
-// the epilogue, the running sums in TMEM and FP64 scores. On 4096 x 4096 F32
-// with 31 x 31, CrossCorr_Norm went from 234 to 214 us, the 3840 x 2160 x 4
-// U16 map with 64 x 64 from 1297 to 1140 us.
+// (staged rows, A operand, energies, maps) slows the MMAs. 4096 x 4096 F32, 31 x 31
+// under the profiler: CrossCorr 253 thousand cycles for 259 steps of 8 MMAs (576
+// cycles), about 930 a step, shared memory 92 percent busy (54 the MMAs, 38 the
+// rest); SqrDistance_Norm 346 thousand, 1290 a step, shared memory 58 percent: with
+// energies the epilogue's chain binds (conversions to FP64, its warps wait as much
+// for the arithmetic pipes as for memory). By the same count a step took 1240 and
+// 1600 with a wait per step, one warp per sub-partition in the epilogue, the running
+// sums in TMEM and FP64 scores. CrossCorr_Norm of that image went from 234 to 208 us
+// (row energies included), the 3840 x 2160 x 4 U16 map with 64 x 64 from 1296 to 1085.
 //
 // Every wait is bounded: a wait that gives up sets the CTA's abort flag, the
 // roles leave their loops, the MMA and TMA threads drain what they issued,
@@ -515,9 +518,8 @@ __device__ __noinline__ void store_slot(const ItemArgs& a, int xl, char* orow,
 // Epilogue of an item, one of two warps of each TMEM sub-partition: warp
 // 4 + 4 h + s takes positions [h S/2, (h + 1) S/2) of lanes 32 s .. 32 s + 31,
 // which have their own 72 columns of the partials (U8: S/2 of every S columns of the
-// ring). One warp is
-// a chain of dependent steps (TMEM round trips, conversions, energies), so
-// the block's time is its latency; with one warp per sub-partition, FP64
+// ring). One warp is a chain of dependent steps (TMEM round trips, conversions,
+// energies), so the block's time is its latency; with one warp per sub-partition, FP64
 // scores of every measure and a wait per 16 columns, the 31 x 31 F32 kernel's
 // step took 1170-1410 cycles here against 580 of the MMAs.
 template <int ELEM, int S, bool IDX, int M>
